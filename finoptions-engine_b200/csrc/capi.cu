@@ -144,7 +144,7 @@ PlanLayout layout_for(const HostPlan& hp, int backward_blocks, int eval_blocks) 
         return at;
     };
     const size_t rows = hp.rows();
-    L.steps = take(sizeof(StepCoef) * std::max<size_t>(hp.intervals(), 1));
+    L.steps = take(sizeof(StepCoef) * align_up(std::max<size_t>(hp.intervals(), 1), kChunkSteps));
     L.events = take(sizeof(NodeEvent) * (hp.intervals() + 1));
     L.row_node = take(sizeof(uint32_t) * rows);
     L.disc_from_later = take(sizeof(double) * rows);
@@ -357,6 +357,7 @@ Error plan_launch(fo_lsm_call_plan* plan) {
     if (plan->run_eval) {
         EvalArgs a{};
         a.plan = plan->dp;
+        a.keys = philox_keys(plan->dp.eval_seed);
         a.records = records;
         a.partials = reinterpret_cast<double2*>(dev + L.eval_partials);
         a.counts = reinterpret_cast<unsigned*>(dev + L.counts);
@@ -715,6 +716,7 @@ Error plan_revalue(fo_lsm_call_plan* plan, const fo_lsm_call_request& q, fo_lsm_
     if (plan->run_eval) {
         EvalArgs a{};
         a.plan = plan->dp;
+        a.keys = philox_keys(plan->dp.eval_seed);
         a.records = reinterpret_cast<const FitRecord*>(dev + L.records);
         a.partials = reinterpret_cast<double2*>(dev + L.eval_partials);
         a.counts = reinterpret_cast<unsigned*>(dev + L.counts);
@@ -766,6 +768,7 @@ Error plan_stopping_rows(fo_lsm_call_plan* plan, uint32_t* rows_out, uint64_t ca
     FO_CUDA_TRY(cudaMemsetAsync(dev + L.itm_counts, 0, sizeof(unsigned) * plan->hp.rows(), s), "reset");
     EvalArgs a{};
     a.plan = plan->dp;
+    a.keys = philox_keys(plan->dp.eval_seed);
     a.records = reinterpret_cast<const FitRecord*>(dev + L.records);
     a.partials = reinterpret_cast<double2*>(dev + L.eval_partials);
     a.counts = reinterpret_cast<unsigned*>(dev + L.counts);

@@ -32,100 +32,70 @@
 namespace fo {
 
 // ----------------------------------------------------------------------------------------------
-// Philox4x32-10 and the path-local stream.
+// Philox4x32-10.
 // ----------------------------------------------------------------------------------------------
 
 constexpr uint32_t kPhiloxM0 = 0xd2511f53u;
 constexpr uint32_t kPhiloxM1 = 0xcd9e8d57u;
 constexpr uint32_t kPhiloxW0 = 0x9e3779b9u;
 constexpr uint32_t kPhiloxW1 = 0xbb67ae85u;
+constexpr int kPhiloxRounds = 10;
 
-// Ten rounds; round r uses key + r * (W0, W1). Output words are the Random123 ordering.
-FO_HD void philox4x32_10(uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3, uint32_t k0, uint32_t k1,
-                         uint32_t out[4]) {
+// The round keys of one seed: round r uses key + r * (W0, W1). A single contract's kernels take them as
+// a launch parameter; the batch kernels, whose launch arguments stay the same from seed to seed, keep
+// them in shared memory, read four at a time.
+struct alignas(16) PhiloxKeys {
+    uint32_t k0[kPhiloxRounds], k1[kPhiloxRounds];
+};
+
+FO_HD PhiloxKeys philox_keys(uint64_t seed) {
+    PhiloxKeys keys;
+    uint32_t k0 = uint32_t(seed), k1 = uint32_t(seed >> 32);
 #pragma unroll
-    for (int r = 0; r < 10; ++r) {
-        // One widening multiply gives both halves of each product.
-        const uint64_t p0 = uint64_t(kPhiloxM0) * c0, p1 = uint64_t(kPhiloxM1) * c2;
-        const uint32_t hi0 = uint32_t(p0 >> 32), lo0 = uint32_t(p0);
-        const uint32_t hi1 = uint32_t(p1 >> 32), lo1 = uint32_t(p1);
-        const uint32_t n0 = hi1 ^ c1 ^ k0;
-        const uint32_t n2 = hi0 ^ c3 ^ k1;
-        c0 = n0;
-        c1 = lo1;
-        c2 = n2;
-        c3 = lo0;
+    for (int r = 0; r < kPhiloxRounds; ++r) {
+        keys.k0[r] = k0;
+        keys.k1[r] = k1;
         k0 += kPhiloxW0;
         k1 += kPhiloxW1;
     }
-    out[0] = c0;
-    out[1] = c1;
-    out[2] = c2;
-    out[3] = c3;
+    return keys;
 }
 
-// Words are consumed as u64 pairs (low word first); one Philox block yields two. The next words
-// wait in a small FIFO (b0 first, up to three). Before every odd-numbered normal (the 1st, 3rd,
-// ...) the stream appends a block while at most one word is queued: the fast path of the sampler
-// takes exactly one word per normal, so in the common case every lane of a warp generates its
-// block at the same normal, even after rejections have shifted lanes against each other within
-// their blocks. A block is also generated whenever a word is wanted from an empty FIFO (only after
-// a rejection). Blocks are generated in counter order and words leave in order, so a path's word
-// sequence does not depend on when its blocks are generated.
-struct PathStream {
-    uint32_t k0, k1, domain, path;
-    uint64_t next_block;
-    uint64_t b0, b1, b2;
-    uint32_t count;      // queued words
-    uint32_t remaining;  // normals left in the budget
-    uint32_t drawn;      // normals begun
-
-    FO_HD void init(uint64_t seed, uint32_t domain_, uint32_t path_, uint32_t budget) {
-        k0 = uint32_t(seed);
-        k1 = uint32_t(seed >> 32);
-        domain = domain_;
-        path = path_;
-        next_block = 0;
-        b0 = b1 = b2 = 0;
-        count = 0;
-        remaining = budget;
-        drawn = 0;
+// Blocks block .. block + N - 1 of a path's stream, N side by side: counter [block_lo, block_hi,
+// path, domain], output words in the Random123 ordering, paired low word first into the u64 words
+// that the sampler consumes.
+template <int N>
+FO_HD void philox_blocks(uint64_t block, uint32_t path, uint32_t domain, const PhiloxKeys& keys,
+                         uint64_t (&words)[2 * N]) {
+    uint32_t c[N][4];
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        c[i][0] = uint32_t(block + i);
+        c[i][1] = uint32_t((block + i) >> 32);
+        c[i][2] = path;
+        c[i][3] = domain;
     }
-    // Appends one block; requires count <= 1.
-    FO_HD void append_block() {
-        uint32_t w[4];
-        philox4x32_10(uint32_t(next_block), uint32_t(next_block >> 32), path, domain, k0, k1, w);
-        next_block += 1;
-        const uint64_t n0 = uint64_t(w[0]) | (uint64_t(w[1]) << 32);
-        const uint64_t n1 = uint64_t(w[2]) | (uint64_t(w[3]) << 32);
-        if (count == 0) {
-            b0 = n0;
-            b1 = n1;
-        } else {
-            b1 = n0;
-            b2 = n1;
+#pragma unroll
+    for (int r = 0; r < kPhiloxRounds; ++r) {
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            // One widening multiply gives both halves of each product.
+            const uint64_t p0 = uint64_t(kPhiloxM0) * c[i][0], p1 = uint64_t(kPhiloxM1) * c[i][2];
+            c[i][0] = uint32_t(p1 >> 32) ^ c[i][1] ^ keys.k0[r];
+            c[i][1] = uint32_t(p1);
+            c[i][2] = uint32_t(p0 >> 32) ^ c[i][3] ^ keys.k1[r];
+            c[i][3] = uint32_t(p0);
         }
-        count += 2;
     }
-    FO_HD uint64_t next_u64() {
-        if (count == 0) append_block();
-        const uint64_t v = b0;
-        b0 = b1;
-        b1 = b2;
-        count -= 1;
-        return v;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        words[2 * i] = uint64_t(c[i][0]) | (uint64_t(c[i][1]) << 32);
+        words[2 * i + 1] = uint64_t(c[i][2]) | (uint64_t(c[i][3]) << 32);
     }
-    FO_HD bool begin_normal() {
-        if (remaining == 0) return false;
-        remaining -= 1;
-        if ((drawn & 1u) == 0 && count <= 1) append_block();
-        drawn += 1;
-        return true;
-    }
-};
+}
 
 // ----------------------------------------------------------------------------------------------
-// ZIGNOR standard normals. Tables live in shared memory on the device (257 + 257 doubles).
+// ZIGNOR standard normals: the layer constants and bit-level conversions (lsm_normals.cuh samples).
 // ----------------------------------------------------------------------------------------------
 
 enum NormalStatus : int { kNormalOk = 0, kNormalBudget = 1, kNormalRejection = 2 };
@@ -202,95 +172,6 @@ FO_HD bool fo_isfinite(double x) {
 #endif
 }
 
-// Tail beyond R (random/normal.rs:50-63), out of line: reached by about one normal in 4000.
-template <typename Tables>
-#if defined(__CUDACC__)
-__host__ __device__ __noinline__
-#else
-inline
-#endif
-int zig_sample_tail(PathStream& s, const Tables& t, double unit, double* out) {
-    const double r = t.r();
-    for (int jt = 0; jt < kMaxRejectionIterations; ++jt) {
-        const double ox = bits_to_double(((s.next_u64() >> 12) & kFractionMask) | kExponent0) -
-                          (1.0 - 1.1102230246251565e-16);
-        const double x = fo_log(ox) / r;
-        const double oy = bits_to_double(((s.next_u64() >> 12) & kFractionMask) | kExponent0) -
-                          (1.0 - 1.1102230246251565e-16);
-        const double y = fo_log(oy);
-        if (-2.0 * y >= x * x) {
-            *out = unit < 0.0 ? x - r : r - x;
-            return kNormalOk;
-        }
-    }
-    return kNormalRejection;
-}
-
-// The rejection loop (random/normal.rs:66-91) from its second pass on, or from the tail, out of line:
-// few normals get here (the tail layer, or a wedge rejection followed by a fast rejection).
-template <typename Tables>
-#if defined(__CUDACC__)
-__host__ __device__ __noinline__
-#else
-inline
-#endif
-int zig_sample_rest(PathStream& s, const Tables& t, int index, double unit, double value, double* out) {
-    for (int it = 0; it < kMaxRejectionIterations - 1; ++it) {
-        if (index == 0) return zig_sample_tail(s, t, unit, out);
-        const double u = double(s.next_u64() >> 11) * (1.0 / 9007199254740992.0);
-        const double ordinate = t.f(index + 1) + (t.f(index) - t.f(index + 1)) * u;
-        if (ordinate < fo_exp(-0.5 * value * value)) {
-            *out = value;
-            return kNormalOk;
-        }
-        const uint64_t bits = s.next_u64();
-        index = int(bits & 0xff);
-        unit = zig_symmetric_unit(bits);
-        value = unit * t.x(index);
-        if (fo_fabs(value) < t.x(index + 1)) {
-            *out = value;
-            return kNormalOk;
-        }
-    }
-    return kNormalRejection;
-}
-
-// One standard normal (random/normal.rs:96-109). The fast test accepts 98.5% of draws; the first wedge
-// test and its redraw are straight-line code, so a warp whose lanes reject at the same normal
-// runs them once; the tail and any further rejection run out of line on a copy of the stream.
-template <typename Tables>
-FO_HD int zig_sample(PathStream& s, const Tables& t, double* out) {
-    if (!s.begin_normal()) return kNormalBudget;
-    uint64_t bits = s.next_u64();
-    int index = int(bits & 0xff);
-    double unit = zig_symmetric_unit(bits);
-    double value = unit * t.x(index);
-    if (fo_fabs(value) < t.x(index + 1)) {
-        *out = value;
-        return kNormalOk;
-    }
-    if (index != 0) {
-        const double u = double(s.next_u64() >> 11) * (1.0 / 9007199254740992.0);
-        const double ordinate = t.f(index + 1) + (t.f(index) - t.f(index + 1)) * u;
-        if (ordinate < fo_exp(-0.5 * value * value)) {
-            *out = value;
-            return kNormalOk;
-        }
-        bits = s.next_u64();
-        index = int(bits & 0xff);
-        unit = zig_symmetric_unit(bits);
-        value = unit * t.x(index);
-        if (fo_fabs(value) < t.x(index + 1)) {
-            *out = value;
-            return kNormalOk;
-        }
-    }
-    PathStream copy = s;
-    const int status = zig_sample_rest(copy, t, index, unit, value, out);
-    s = copy;
-    return status;
-}
-
 // ----------------------------------------------------------------------------------------------
 // Division by a divisor used many times (the strike, a fitted scale): the reciprocal y = 1/b is
 // formed once and each quotient takes Markstein's correction step (P. Markstein, "Computation of
@@ -310,6 +191,15 @@ struct Divisor {
 FO_HD Divisor make_divisor(double b) {
     const double m = fo_fabs(b);
     return Divisor{b, (m > 0x1p-960 && m < 0x1p960) ? 1.0 / b : 0.0};
+}
+
+// divide for a > d.b > 0 with d.inv != 0: the same quotient without the range checks. An a above
+// the corrected range loses nothing (the residual only underflows for small a); where q0 overflows
+// the result is not finite, and the caller divides.
+FO_HD double divide_above(double a, const Divisor& d) {
+    const double q0 = a * d.inv;
+    const double r = fo_fma(-d.b, q0, a);
+    return fo_fma(r, d.inv, q0);
 }
 
 FO_HD double divide(double a, const Divisor& d) {
@@ -845,30 +735,83 @@ FO_HD bool predict_continuation_d(const Model& m, double predictor, double* out)
     return true;
 }
 
-#ifdef __CUDACC__
-// predict_continuation_d for a model in shared memory that the pass reads at every path: the same
-// operations in the same order, with the fields read through a volatile reference so the compiler
-// loads them per path (broadcast shared-memory loads) instead of holding the 14 of them in
-// registers across the pass; the registers go to resident CTAs instead.
-template <int D>
-__device__ __forceinline__ bool predict_continuation_shared(const FitModel* model, double predictor, double* out) {
-    const volatile FitModel& m = *model;
-    if (!fo_isfinite(predictor)) return false;
-    const double z = D == 0 ? 0.0 : divide(predictor - m.mean, Divisor{m.scale, m.inv_scale});
-    double prediction = m.coef[0];
-    double previous = 0.0, current = 1.0;
-#pragma unroll
-    for (int j = 0; j < D; ++j) {
-        const double next = fo_fma(z - m.alpha[j], current, -m.beta[j] * previous);
-        prediction = fo_fma(m.coef[j + 1], next, prediction);
-        previous = current;
-        current = next;
-    }
-    if (!fo_isfinite(prediction)) return false;
-    *out = prediction;
-    return true;
+// The exercise rule of a fitted row as the passes over paths apply it: with d = spot - strike (the
+// intrinsic value, exact near the strike), z = d * slope + shift is the standardised moneyness
+// (spot / strike - mean) / scale, and the continuation is its polynomial in powers of z. Exercise
+// where d > 0 and d exceeds the continuation. One fma standardises and D evaluate, against three to
+// divide by the strike, three more to divide by the scale and 4 D for the basis recurrence; the
+// rounding of z is of the order of ulp(max(|z|, 1)), where that of spot / strike is magnified by
+// 1 / scale, so the continuation is at least as close to the fitted polynomial.
+//
+// The rule covers spots below kRuleSpotLimit of rows for which no intermediate can overflow there
+// (the bound is evaluated in make_exercise_rule). `general` marks every other row that needs more
+// than this test (no training support; extreme strikes, scales or coefficients): it is decided by
+// predict_continuation. Rows that never exercise have the continuation +infinity.
+struct alignas(16) ExerciseRule {
+    double slope, shift;
+    double c[kMaxColumns];
+    int32_t general;
+    int32_t pad;
+};
+constexpr double kRuleSpotLimit = 0x1p200;
+
+FO_HD ExerciseRule never_exercise() {
+    ExerciseRule r{};
+    r.c[0] = bits_to_double(uint64_t(0x7ff) << 52);
+    return r;
 }
-#endif
+
+FO_HD ExerciseRule make_exercise_rule(const FitModel& m, int degree, double strike) {
+    ExerciseRule r{};
+    // Powers of z from the basis p_{j+1} = (z - alpha_j) p_j - beta_j p_{j-1}.
+    double previous[kMaxColumns], current[kMaxColumns];
+#pragma unroll
+    for (int i = 0; i < kMaxColumns; ++i) {
+        previous[i] = 0.0;
+        current[i] = i == 0 ? 1.0 : 0.0;
+        r.c[i] = i == 0 ? m.coef[0] : 0.0;
+    }
+#pragma unroll
+    for (int j = 0; j < kMaxDegree; ++j) {
+        if (j >= degree) break;
+        double next[kMaxColumns];
+#pragma unroll
+        for (int i = 0; i < kMaxColumns; ++i) {
+            const double shifted = i > 0 ? current[i - 1] : 0.0;
+            next[i] = fo_fma(-m.beta[j], previous[i], fo_fma(-m.alpha[j], current[i], shifted));
+            r.c[i] = fo_fma(m.coef[j + 1], next[i], r.c[i]);
+        }
+#pragma unroll
+        for (int i = 0; i < kMaxColumns; ++i) {
+            previous[i] = current[i];
+            current[i] = next[i];
+        }
+    }
+    if (degree > 0) {
+        r.slope = 1.0 / (strike * m.scale);
+        r.shift = (1.0 - m.mean) / m.scale;
+    }
+    const double reach = fo_fma(kRuleSpotLimit, r.slope, fo_fabs(r.shift));
+    double bound = 0.0;
+#pragma unroll
+    for (int i = kMaxColumns - 1; i >= 0; --i) bound = fo_fma(bound, reach, fo_fabs(r.c[i]));
+    const bool plain = strike > 0x1p-100 && strike < 0x1p100 && m.scale > 0x1p-100 && m.scale < 0x1p100 &&
+                       fo_isfinite(bound);
+    r.general = plain ? 0 : 1;
+    return r;
+}
+
+// The continuation of a spot `excess` above the strike; Rule is ExerciseRule, or a volatile one in
+// shared memory that a pass reads at every path instead of holding it in registers.
+template <int D, typename Rule>
+FO_HD double rule_continuation(const Rule& r, double excess) {
+    if (D == 0) return r.c[0];
+    const double z = fo_fma(excess, r.slope, r.shift);
+    double p = r.c[D];
+#pragma unroll
+    for (int k = D - 1; k >= 0; --k) p = fo_fma(p, z, r.c[k]);
+    return p;
+}
 
 // ----------------------------------------------------------------------------------------------
 // Rank and two-norm condition diagnostic: one-sided Jacobi SVD of the <= 5x5 upper-triangular

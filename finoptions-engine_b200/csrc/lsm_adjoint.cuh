@@ -39,8 +39,11 @@ struct GreekSums {
 // Segment bookkeeping of one evaluation path: seg = cash dividends applied so far; growth[s] =
 // product of the step factors of segment s; sens[s] = its sum of dP/du_i-weights for sigma; pre[j]
 // = the state before cash j, above[j] = whether that state exceeded the amount, node[j] its node.
+// The open segment's pair is in `factor` and `weight`: every step updates it, and an array element
+// at a running index would go through local memory.
 struct PathAdjoint {
     int seg;
+    double factor, weight;
     double growth[kMaxGreekDividends + 1];
     double sens[kMaxGreekDividends + 1];
     double pre[kMaxGreekDividends];
@@ -49,27 +52,31 @@ struct PathAdjoint {
 
     __device__ void reset() {
         seg = 0;
-        growth[0] = 1.0;
-        sens[0] = 0.0;
+        factor = 1.0;
+        weight = 0.0;
     }
     __device__ void step(double g, double sens_term) {
-        growth[seg] *= g;
-        sens[seg] += sens_term;
+        factor *= g;
+        weight += sens_term;
     }
     __device__ void cash(uint32_t at, double before, double amount) {
         if (seg >= kMaxGreekDividends) return;
+        growth[seg] = factor;
+        sens[seg] = weight;
         pre[seg] = before;
         above[seg] = before > amount;
         node[seg] = at;
         seg += 1;
-        growth[seg] = 1.0;
-        sens[seg] = 0.0;
+        factor = 1.0;
+        weight = 0.0;
     }
     // A path stops at `at` with observed state s_obs, payoff pay = (s_obs - K) * ad > 0. Adds its
     // delta, vega (sens scaled by sens_scale), log-discount and dividend contributions.
     __device__ void stop(GreekSums& acc, uint32_t at, double s_obs, double pay, double ad, bool terminal, int policy,
-                         double sens_scale) const {
+                         double sens_scale) {
         if (!(pay > 0.0)) return;
+        growth[seg] = factor;
+        sens[seg] = weight;
         int s = seg;
         double a_end = ad, s_end = s_obs;
         if (terminal && s > 0 && node[s - 1] == at) {

@@ -91,16 +91,6 @@ enum FitFailKind : int32_t {
 // Strikes evaluated together by one evaluation thread (groups with more run several passes).
 constexpr int kEvalStrikes = 8;
 
-// The part of a fitted row the evaluation reads, staged in shared memory per (strike, row).
-struct PolicyRule {
-    double mean, scale, inv_scale;
-    double alpha[kMaxDegree];
-    double beta[kMaxDegree];
-    double coef[kMaxColumns];
-    int32_t kind;
-    int32_t pad;
-};
-
 // Shared memory the evaluation may spend on staged rules; larger groups read them from HBM.
 constexpr size_t kEvalRuleSmemBytes = 96 * 1024;
 
@@ -148,6 +138,7 @@ struct BatchArgs {
     double* slab;
     double* values;
     FitRecord* records;
+    ExerciseRule* rules;       // [records]: the row's rule as the evaluation applies it
     GroupStatus* group_status;
     ProblemStatus* problem_status;
     unsigned* counts;          // [problems * 2]: early, expiry

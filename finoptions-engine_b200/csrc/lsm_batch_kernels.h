@@ -21,9 +21,12 @@ struct BatchTuning {
     int phases = 0;       // 1: one kernel per item kind and a summary kernel instead of one launch
 };
 
-// Shared memory of the staged fitted rules: `strikes` x rule_rows PolicyRules, or with the Greeks
-// one strike's rules and its per-row stopping counts.
-size_t persistent_rule_bytes(int strikes, bool greeks, uint32_t rule_rows);
+// Shared memory of the staged exercise rules: rule_rows x `strikes` of them and one word per row
+// (whether the row needs its records), or with the Greeks one strike's rules and its per-row stopping
+// counts.
+inline size_t persistent_rule_bytes(int strikes, bool greeks, uint32_t rule_rows) {
+    return (sizeof(ExerciseRule) * size_t(greeks ? 1 : strikes) + sizeof(unsigned)) * rule_rows;
+}
 // One persistent launch over the queue q, in two steps so that the second can be captured into a
 // CUDA graph: the kernel instance for the launch shape, its dynamic shared memory and its grid
 // (resident CTAs, at most one per item), then the launch itself on `stream`.

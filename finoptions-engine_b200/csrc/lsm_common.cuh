@@ -1,5 +1,5 @@
 // lsm_common.cuh - device building blocks shared by the single-contract and batch LSM kernels:
-// ZIGNOR tables in shared memory, the seeded path simulation with event phases, deterministic
+// the seeded path simulation with event phases, deterministic
 // warp / CTA / grid reductions, the exercise rule and the in-the-money power-sum accumulator.
 #pragma once
 
@@ -7,29 +7,11 @@
 #include <stdint.h>
 
 #include "lsm_device.cuh"
+#include "lsm_normals.cuh"
 
 namespace fo {
 
-static __constant__ uint64_t c_zig_x[257] = FO_ZIG_NORM_X_BITS;
-static __constant__ uint64_t c_zig_f[257] = FO_ZIG_NORM_F_BITS;
-
 constexpr unsigned long long kNone = ~0ull;
-
-__device__ __forceinline__ void load_zig_tables(double* sx, double* sf) {
-    for (int i = threadIdx.x; i < 257; i += blockDim.x) {
-        sx[i] = bits_to_double(c_zig_x[i]);
-        sf[i] = bits_to_double(c_zig_f[i]);
-    }
-    __syncthreads();
-}
-
-__device__ __forceinline__ SmemZig make_zig(const double* sx, const double* sf) {
-    SmemZig z;
-    z.xs = sx;
-    z.fs = sf;
-    z.rr = bits_to_double(FO_ZIG_NORM_R_BITS);
-    return z;
-}
 
 // ---------------------------------------------------------------------------------------------
 // Seeded path simulation
@@ -42,40 +24,92 @@ struct SimResult {
     double normal;
 };
 
-// Simulates one path; calls store(row, value) at every observation. Mirrors simulate_one_seeded
-// (seeded.rs:399-459) including the terminal-dividend phase order.
-template <typename Store>
-__device__ __forceinline__ SimResult simulate_path(const DevicePlan& plan, const SmemZig& zig, uint64_t seed,
-                                                   uint32_t domain, uint32_t path, Store&& store) {
-    PathStream s;
-    s.init(seed, domain, path, plan.intervals);
+// One GBM step by a growth factor: the state after it, or false for a non-finite transition. A finite
+// product of non-negative factors has a high word below the exponent's, so one integer comparison
+// passes it; the absorbed state (0 times an overflowed factor) and the failures take the branch.
+__device__ __forceinline__ bool gbm_step(double spot, double growth, double* next) {
+    *next = spot * growth;
+    if (uint32_t(__double2hiint(*next)) < 0x7ff00000u) return true;
+    if (spot == 0.0) *next = 0.0;
+    return fo_isfinite(*next);
+}
+
+// Simulates one path; calls store(row, value) at every observation, step(i, coefficients, normal,
+// growth) after every interval and cash(node, state before, amount) after every cash dividend.
+// Mirrors simulate_one_seeded (seeded.rs:399-459) including the terminal-dividend phase order.
+// kInline: a chunk's four steps are unrolled; otherwise (an observer of hundreds of instructions) they
+// loop, with the growth factors parked in shared memory. Four steps' normals and growth
+// factors are formed side by side (they do not depend on the state): the four exponentials share
+// the polynomial's constants, which a kernel of this register budget otherwise sets up again for
+// each of them (25 of a step's 62 instructions measured).
+struct IgnoreStep {
+    __device__ __forceinline__ void operator()(uint32_t, const StepCoef&, double, double) const {}
+};
+struct IgnoreCash {
+    __device__ __forceinline__ void operator()(uint32_t, double, double) const {}
+};
+
+template <bool kInline = true, int T, typename Store, typename Step = IgnoreStep, typename Cash = IgnoreCash>
+__device__ __forceinline__ SimResult simulate_path(const DevicePlan& plan, NormalSmem<T>& normals,
+                                                   const PhiloxKeys& keys, uint32_t domain, uint32_t path,
+                                                   Store&& store, Step&& step = Step{}, Cash&& cash = Cash{}) {
+    const uint32_t intervals = plan.intervals;
+    NormalStream<T> s;
+    s.init(normals, domain, path);
     double spot = plan.sim_start;
     SimResult r{0, 0, 0.0, 0.0};
     if (plan.row_node[0] == 0) store(0, spot);
-    for (uint32_t i = 0; i < plan.intervals; ++i) {
-        double z = 0.0;
-        const int status = zig_sample(s, zig, &z);
-        if (status != kNormalOk) {
-            r.code = status;
+    for (uint32_t i = 0; i < intervals; i += kChunkNormals) {
+        double z[kChunkNormals], growth[kChunkNormals];
+        if (!s.next4(keys, i, intervals, z)) {
+            r.code = kNormalRejection;
             r.interval = int(i);
             return r;
         }
-        const StepCoef c = plan.steps[i];
-        const double next = gbm_advance(spot, c.diffusion, c.log_drift, z);
-        if (!fo_isfinite(next)) {
-            r.code = 3;
-            r.interval = int(i);
-            r.spot = spot;
-            r.normal = z;
-            return r;
+#pragma unroll
+        for (uint32_t j = 0; j < kChunkNormals; ++j) {
+            const StepCoef c = plan.steps[i + j];  // padded to whole chunks
+            growth[j] = fo_exp(fo_fma(c.diffusion, z[j], c.log_drift));
         }
-        spot = next;
-        const NodeEvent ev = plan.events[i + 1];
-        const bool dividend = (ev.flags & kEventDividend) != 0;
-        const bool terminal = (ev.flags & kEventTerminal) != 0;
-        if (dividend && terminal) spot = apply_cash_dividend(plan.policy, ev.dividend_amount, spot);
-        if (ev.row >= 0) store(ev.row, spot);
-        if (dividend && !terminal) spot = apply_cash_dividend(plan.policy, ev.dividend_amount, spot);
+        if constexpr (!kInline) {
+#pragma unroll
+            for (uint32_t j = 0; j < kChunkNormals; ++j) normals.parked[j][threadIdx.x] = growth[j];
+        }
+        const auto advance = [&](uint32_t j, double factor, double normal) -> bool {
+            double next;
+            if (!gbm_step(spot, factor, &next)) {
+                r.code = 3;
+                r.interval = int(i + j);
+                r.spot = spot;
+                r.normal = normal;
+                return false;
+            }
+            step(i + j, plan.steps[i + j], normal, factor);
+            spot = next;
+            const NodeEvent ev = plan.events[i + j + 1];
+            const auto pay = [&] {
+                const double before = spot;
+                spot = apply_cash_dividend(plan.policy, ev.dividend_amount, before);
+                cash(i + j + 1, before, ev.dividend_amount);
+            };
+            const int32_t phase = ev.flags & (kEventDividend | kEventTerminal);
+            if (phase == (kEventDividend | kEventTerminal)) pay();
+            if (ev.row >= 0) store(ev.row, spot);
+            if (phase == kEventDividend) pay();
+            return true;
+        };
+        if constexpr (kInline) {
+#pragma unroll
+            for (uint32_t j = 0; j < kChunkNormals; ++j) {
+                if (j > 0 && i + j >= intervals) return r;
+                if (!advance(j, growth[j], z[j])) return r;
+            }
+        } else {
+            const uint32_t steps = min(kChunkNormals, intervals - i);
+#pragma unroll 1
+            for (uint32_t j = 0; j < steps; ++j)
+                if (!advance(j, normals.parked[j][threadIdx.x], s.normal(i + j))) return r;
+        }
     }
     return r;
 }
@@ -226,13 +260,32 @@ __device__ __forceinline__ bool exercise_rule(int tie_rule, double intrinsic, do
     return tie_rule == 0 ? intrinsic > continuation : intrinsic >= continuation;
 }
 
+// Whether a spot is below kRuleSpotLimit, by its high word (spots are not negative).
+__device__ __forceinline__ bool within_rule(double spot) { return uint32_t(__double2hiint(spot)) < 0x4c700000u; }
+static_assert(kRuleSpotLimit == 0x1p200, "high word 0x4c700000");
+
+// The decision of an in-the-money spot that the row's ExerciseRule does not cover. No ordinary market
+// gets here, but it stays in line: a call in a path loop costs the loop's registers.
+enum Decision : int { kDecideContinue = 0, kDecideExercise = 1, kDecideNonFinite = 2 };
+
+template <int D>
+__device__ __forceinline__ int decide_general(const FitModel* model, double spot, double strike, int tie_rule) {
+    double continuation;
+    if (!predict_continuation_d<D>(*model, divide(spot, make_divisor(strike)), &continuation)) return kDecideNonFinite;
+    return exercise_rule(tie_rule, spot - strike, continuation) ? kDecideExercise : kDecideContinue;
+}
+
 struct RowSums {
     double acc[kSlots];
 };
 
-__device__ __forceinline__ void accumulate_itm(RowSums& r, double x, double y, double pivot) {
+// A non-negative number's finiteness by its high word (a NaN or an infinity has it at the exponent's
+// maximum or, with the sign set, above).
+__device__ __forceinline__ bool finite_nonnegative(double v) { return uint32_t(__double2hiint(v)) < 0x7ff00000u; }
+
+// The sums of one in-the-money path but for its count (acc[0]).
+__device__ __forceinline__ void accumulate_moments(RowSums& r, double x, double y, double pivot) {
     const double t = x - pivot;
-    r.acc[0] += 1.0;
     double pw = t;
     r.acc[kPowerSums] += y;
 #pragma unroll
@@ -241,6 +294,11 @@ __device__ __forceinline__ void accumulate_itm(RowSums& r, double x, double y, d
         if (k < kResponseSums) r.acc[kPowerSums + k] = fo_fma(y, pw, r.acc[kPowerSums + k]);
         pw *= t;
     }
+}
+
+__device__ __forceinline__ void accumulate_itm(RowSums& r, double x, double y, double pivot) {
+    r.acc[0] += 1.0;
+    accumulate_moments(r, x, y, pivot);
 }
 
 // The halves of accumulate_itm: count and T_1..T_8 of t = x - pivot (they do not depend on the

@@ -13,6 +13,7 @@ struct StepCoef {
     double log_drift;
     double diffusion;
 };
+constexpr uint32_t kChunkSteps = 4;  // steps whose normals and growth factors are formed together
 
 // Event phases at grid node n >= 1 (crates/finoptions-sim/src/path.rs:422-472): the observation
 // row recorded at the node (-1 if none) and an optional cash dividend. At the terminal
@@ -100,23 +101,13 @@ struct DevicePlan {
     uint64_t train_paths, eval_paths;
     uint64_t train_seed, eval_seed;
     uint32_t train_domain, eval_domain;
-    const StepCoef* steps;     // [intervals]
+    const StepCoef* steps;     // [intervals], padded to a multiple of kChunkSteps
     const NodeEvent* events;   // [intervals + 1] (index by node; node 0 unused)
     const uint32_t* row_node;  // [rows]
     const double* disc_from_later;  // [rows]: exp(L[later] - L[node]) for positive exercise rows
     const double* disc_to_origin;   // [rows]: exp(L[node])
     const double* escrow_cash;      // [rows]: prepaid cash added to observations (escrowed)
     double origin_discount;    // exp(L[last processed node]) applied before the origin mean
-};
-
-// Device tables for ZIGNOR, held in shared memory.
-struct SmemZig {
-    const double* xs;
-    const double* fs;
-    double rr;
-    FO_D double x(int i) const { return xs[i]; }
-    FO_D double f(int i) const { return fs[i]; }
-    FO_D double r() const { return rr; }
 };
 
 }  // namespace fo

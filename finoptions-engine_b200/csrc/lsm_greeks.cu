@@ -23,16 +23,10 @@
 #include "lsm_adjoint.cuh"
 #include "lsm_common.cuh"
 #include "lsm_device.cuh"
+#include "lsm_evaluate.cuh"
 #include "lsm_kernels.h"
 
 namespace fo {
-
-struct GreeksEvalRow {
-    FitModel model;
-    int32_t kind;
-    int32_t pad;
-    double discount;
-};
 
 template <int D>  // == plan.degree
 __global__ void __launch_bounds__(kEvalThreads, 4) evaluate_greeks_kernel(EvalArgs a, GreeksArgs gk) {
@@ -41,29 +35,18 @@ __global__ void __launch_bounds__(kEvalThreads, 4) evaluate_greeks_kernel(EvalAr
     __shared__ dd gtot[kGreekSlots];
     const DevicePlan& plan = a.plan;
     const uint32_t rows = plan.rows;
-    double* sx = reinterpret_cast<double*>(greeks_smem_raw);
-    double* sf = sx + 257;
-    double* red = sf + 257;                                             // [32 * 2]
-    GreeksEvalRow* rules = reinterpret_cast<GreeksEvalRow*>(red + 64);  // [rows]
+    __shared__ NormalSmem<kEvalThreads> normals;
+    __shared__ double red[32 * 2];
+    EvalRow* rules = reinterpret_cast<EvalRow*>(greeks_smem_raw);             // [rows]
     unsigned* counts = reinterpret_cast<unsigned*>(rules + rows);       // [rows]
     unsigned* itm_counts = counts + rows;                               // [rows]
+    const double K = plan.strike;
     for (uint32_t r = threadIdx.x; r < rows; r += blockDim.x) {
-        GreeksEvalRow er;
-        if (r + 1 < rows) {
-            er.model = a.records[r].model;
-            er.kind = a.records[r].kind;
-        } else {
-            er.kind = kRuleNone;
-        }
-        er.discount = plan.disc_to_origin[r];
-        rules[r] = er;
+        rules[r] = make_eval_row(plan, a.records, r);
         counts[r] = 0;
         itm_counts[r] = 0;
     }
-    load_zig_tables(sx, sf);
-    const SmemZig zig = make_zig(sx, sf);
-    const double K = plan.strike;
-    const Divisor Kd = make_divisor(K);
+    load_normal_tables(normals);
     const uint64_t P = plan.eval_paths;
     const uint32_t last = rows - 1;
     double sum = 0.0, sumsq = 0.0;
@@ -71,83 +54,47 @@ __global__ void __launch_bounds__(kEvalThreads, 4) evaluate_greeks_kernel(EvalAr
     gs.reset();
     for (uint64_t p = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; p < P; p += uint64_t(gridDim.x) * blockDim.x) {
         bool active = true;
-        double payoff = 0.0;
+        double payoff = 0.0, held = 0.0;  // the payoff and the state it was taken at
+        uint32_t stop_row = 0;
         PathAdjoint adj;
         adj.reset();
         auto observe = [&](int row, double spot) {
             if (!active) return;
-            const GreeksEvalRow& er = rules[row];
+            const EvalRow& er = rules[row];
             if (uint32_t(row) == last) {
                 const double d = spot - K;
                 payoff = (d > 0.0 ? d : 0.0) * er.discount;
                 if (!fo_isfinite(payoff)) atomicMin(&a.status->eval_terminal_fail, (unsigned long long)p);
                 active = false;
-                atomicAdd(&counts[row], 1u);
-                adj.stop(gs, plan.row_node[row], spot, payoff, er.discount, true, plan.policy, 1.0);
+                held = spot;
+                stop_row = last;
                 return;
             }
-            if (er.kind == kRuleNoSupport) {
-                if (spot > K) atomicAdd(&itm_counts[row], 1u);
-                return;
-            }
-            if (er.kind != kRuleRegression || !(spot > K)) return;
-            const double intrinsic = spot - K;
-            double continuation;
-            if (!predict_continuation_d<D>(er.model, divide(spot, Kd), &continuation)) {
-                atomicMin(&a.status->eval_fail, ((unsigned long long)row << 33) | (p << 1));
-                return;
-            }
-            if (exercise_rule(plan.tie_rule, intrinsic, continuation)) {
-                payoff = intrinsic * er.discount;
+            const double excess = spot - K;
+            if (!(excess > 0.0)) return;
+            if (decide_row<D>(plan, a.records, a.status, er.rule, uint32_t(row), p, spot, excess, itm_counts)) {
+                payoff = excess * er.discount;
                 if (!fo_isfinite(payoff))
                     atomicMin(&a.status->eval_fail, ((unsigned long long)row << 33) | (p << 1) | 1ull);
                 active = false;
-                atomicAdd(&counts[row], 1u);
-                adj.stop(gs, plan.row_node[row], spot, payoff, er.discount, false, plan.policy, 1.0);
+                held = spot;
+                stop_row = uint32_t(row);
             }
         };
-        // The path: simulate_path's arithmetic and event phases, with the segment bookkeeping.
-        PathStream s;
-        s.init(plan.eval_seed, plan.eval_domain, uint32_t(p), plan.intervals);
-        double spot = plan.sim_start;
-        if (plan.row_node[0] == 0) observe(0, spot);
-        bool failed = false;
-        for (uint32_t i = 0; i < plan.intervals; ++i) {
-            double z = 0.0;
-            if (zig_sample(s, zig, &z) != kNormalOk) {
-                failed = true;
-                break;
-            }
-            const StepCoef c = plan.steps[i];
-            double next = 0.0;
-            double g = 1.0;
-            if (spot != 0.0) {
-                g = fo_exp(fo_fma(c.diffusion, z, c.log_drift));
-                next = spot * g;
-            }
-            if (!fo_isfinite(next)) {
-                failed = true;
-                break;
-            }
+        const auto step = [&](uint32_t i, const StepCoef&, double z, double g) {
             if (active) adj.step(g, z * gk.sqrt_dt[i] - gk.sigma * gk.dt[i]);
-            spot = next;
-            const uint32_t at = i + 1;
-            const NodeEvent ev = plan.events[at];
-            const bool dividend = (ev.flags & kEventDividend) != 0;
-            const bool terminal = (ev.flags & kEventTerminal) != 0;
-            if (dividend && terminal) {
-                const double before = spot;
-                spot = apply_cash_dividend(plan.policy, ev.dividend_amount, before);
-                if (active) adj.cash(at, before, ev.dividend_amount);
-            }
-            if (ev.row >= 0) observe(ev.row, spot);
-            if (dividend && !terminal) {
-                const double before = spot;
-                spot = apply_cash_dividend(plan.policy, ev.dividend_amount, before);
-                if (active) adj.cash(at, before, ev.dividend_amount);
-            }
+        };
+        const auto cash = [&](uint32_t at, double before, double amount) {
+            if (active) adj.cash(at, before, amount);
+        };
+        const SimResult r = simulate_path<false>(plan, normals, a.keys, plan.eval_domain, uint32_t(p), observe, step, cash);
+        if (r.code != 0) atomicMin(&a.status->eval_sim_fail, (unsigned long long)p);
+        // The backward recurrence after the path, where its sums are not live through the path's loop.
+        if (!active) {
+            atomicAdd(&counts[stop_row], 1u);
+            adj.stop(gs, plan.row_node[stop_row], held, payoff, rules[stop_row].discount, stop_row == last,
+                     plan.policy, 1.0);
         }
-        if (failed) atomicMin(&a.status->eval_sim_fail, (unsigned long long)p);
         sum += payoff;
         sumsq += payoff * payoff;
     }
@@ -174,14 +121,14 @@ __global__ void __launch_bounds__(32 * kGreekSlots) finalize_greeks_kernel(const
 }
 
 size_t evaluate_greeks_smem_bytes(uint32_t rows) {
-    return sizeof(double) * (257 * 2 + 64) + sizeof(GreeksEvalRow) * rows + sizeof(unsigned) * 2 * rows;
+    return sizeof(EvalRow) * rows + sizeof(unsigned) * 2 * rows;
 }
 
 template <int D>
 static cudaError_t launch_evaluate_greeks_d(const EvalArgs& args, const GreeksArgs& greeks, int blocks,
                                             cudaStream_t stream) {
     const size_t smem = evaluate_greeks_smem_bytes(args.plan.rows);
-    if (smem > 48 * 1024) {
+    if (smem > kSmallDynamicSmem) {
         cudaError_t e =
             cudaFuncSetAttribute(evaluate_greeks_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
         if (e != cudaSuccess) return e;

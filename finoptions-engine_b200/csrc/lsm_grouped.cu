@@ -34,7 +34,8 @@ namespace {
 constexpr unsigned long long kNone = ~0ull;
 // Shared memory the persistent launch may spend on staged fitted rules (with three 80-register
 // CTAs per SM, about 57 KB each leaves every CTA resident; more lowers the CTAs per SM).
-constexpr size_t kPersistentRuleSmemBytes = 200 * 1024;
+constexpr size_t kPersistentRuleSmemBytes = 160 * 1024;
+constexpr uint32_t kGreekRuleRows = 1462;  // observation rows of a contract priced with its Greeks
 constexpr int kPersistentMaxCtasPerSm = 3;  // the persistent kernel's launch bounds
 constexpr uint64_t kU32Max = 0xffffffffull;
 
@@ -802,7 +803,7 @@ struct WaveLayout {
     size_t groups, problems, items, group_status, problem_status, summaries;  // read-back region: group_status..summaries
     size_t counters;
     size_t greek_sums;                                                  // (read back, Greeks only)
-    size_t counts, itm_counts, stop_counts, eval_partials, greek_partials, records, values, slab, replay;
+    size_t counts, itm_counts, stop_counts, rules, eval_partials, greek_partials, records, values, slab, replay;
     size_t team_arrive, team_slots;
     size_t out_begin, out_bytes, clear_begin, clear_bytes, total;
 };
@@ -862,6 +863,7 @@ WaveLayout layout_for(const Wave& w, size_t base) {
     L.team_arrive = take(sizeof(unsigned) * P);
     off = align_up(off, 256);
     L.clear_bytes = off - L.clear_begin;
+    L.rules = take(sizeof(ExerciseRule) * w.records);
     L.eval_partials = take(sizeof(double2) * 2 * std::max<uint64_t>(w.partial_slots, 1));
     L.greek_partials = take(w.greeks ? sizeof(double2) * kGreekSlots * w.partial_slots : 0);
     L.replay = take(sizeof(SimFailure));
@@ -1244,7 +1246,7 @@ Error price_groups(fo_executor* ex, const BatchMethod& m, const std::vector<Grou
     for (uint64_t g = 0; g < launchable; ++g) {
         const HostPlan& hp = work[g].hp;
         InputOffsets& o = offsets[g];
-        o.steps = take(sizeof(StepCoef) * std::max<size_t>(hp.steps.size(), 1));
+        o.steps = take(sizeof(StepCoef) * align_up(std::max<size_t>(hp.steps.size(), 1), kChunkSteps));
         o.events = take(sizeof(NodeEvent) * hp.events.size());
         o.row_node = take(sizeof(uint32_t) * hp.rows());
         o.disc_from_later = take(sizeof(double) * hp.rows());
@@ -1281,7 +1283,7 @@ Error price_groups(fo_executor* ex, const BatchMethod& m, const std::vector<Grou
             const uint32_t eval_blocks = eval_blocks_for(hp.eval_paths);
             const uint32_t train_blocks = eval_blocks_for(hp.train_paths);
             const size_t cost = sizeof(double) * (stored + strikes_g) * hp.train_paths +
-                                strikes_g * (rows * (sizeof(FitRecord) + 2 * sizeof(unsigned)) +
+                                strikes_g * (rows * (sizeof(FitRecord) + sizeof(ExerciseRule) + 2 * sizeof(unsigned)) +
                                              size_t(eval_blocks) * sizeof(double2) * (2 + (greeks ? kGreekSlots : 0)) +
                                              sizeof(BatchProblem) + sizeof(ProblemStatus) + sizeof(ProblemSummary) +
                                              sizeof(double) * kGreekSlots + sizeof(uint32_t) + 8) +
@@ -1410,10 +1412,10 @@ Error price_groups(fo_executor* ex, const BatchMethod& m, const std::vector<Grou
                     eval_strikes *= 2;
             const size_t rule_bytes = persistent_rule_bytes(eval_strikes, greeks, max_rows);
             const bool stage = rule_bytes <= kPersistentRuleSmemBytes;
-            if (greeks && !stage)
+            if (greeks && max_rows > kGreekRuleRows)
                 return make_error(FO_ERR_EXECUTION, FO_CODE_CAPACITY_EXCEEDED,
                                   "adjoint Greeks of a batch hold at most " +
-                                      u(kPersistentRuleSmemBytes / (sizeof(PolicyRule) + 4)) +
+                                      u(kGreekRuleRows) +
                                       " observation rows per contract; observed " + u(max_rows));
             // The items are written straight into their region of the pinned staging buffer, which
             // the wave layout sizes for the finest cut (w.item_bound): no per-call allocation or copy.
@@ -1506,6 +1508,7 @@ Error price_groups(fo_executor* ex, const BatchMethod& m, const std::vector<Grou
             a.slab = reinterpret_cast<double*>(dev + L.slab);
             a.values = reinterpret_cast<double*>(dev + L.values);
             a.records = reinterpret_cast<FitRecord*>(dev + L.records);
+            a.rules = reinterpret_cast<ExerciseRule*>(dev + L.rules);
             a.group_status = reinterpret_cast<GroupStatus*>(dev + L.group_status);
             a.problem_status = reinterpret_cast<ProblemStatus*>(dev + L.problem_status);
             a.counts = reinterpret_cast<unsigned*>(dev + L.counts);

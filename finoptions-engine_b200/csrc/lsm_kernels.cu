@@ -21,6 +21,7 @@
 
 #include "lsm_common.cuh"
 #include "lsm_device.cuh"
+#include "lsm_evaluate.cuh"
 #include "lsm_fit_warp.cuh"
 #include "lsm_kernels.h"
 #include "lsm_sync.cuh"
@@ -36,6 +37,8 @@ __device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
+constexpr int kSimulateThreads = 256;
+constexpr int kReplayThreads = 32;
 constexpr int kCombineWarps = kSlots;  // warps 0..15 wait for and combine the CTA partials
 constexpr int kCombineThreads = kCombineWarps * 32;
 
@@ -82,24 +85,25 @@ __device__ __forceinline__ void combine_published(const double2* partials, unsig
 // Normals export
 // ---------------------------------------------------------------------------------------------
 
-__global__ void __launch_bounds__(256) normals_kernel(uint64_t seed, uint32_t domain, uint32_t path_start,
-                                                      uint64_t paths, uint32_t count, double* out,
-                                                      unsigned long long* fail) {
-    __shared__ double sx[257], sf[257];
-    load_zig_tables(sx, sf);
-    const SmemZig zig = make_zig(sx, sf);
+__global__ void __launch_bounds__(kSimulateThreads) normals_kernel(PhiloxKeys keys, uint32_t domain,
+                                                                   uint32_t path_start, uint64_t paths,
+                                                                   uint32_t count, double* out,
+                                                                   unsigned long long* fail) {
+    __shared__ NormalSmem<kSimulateThreads> normals;
+    load_normal_tables(normals);
     for (uint64_t p = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; p < paths;
          p += uint64_t(gridDim.x) * blockDim.x) {
-        PathStream s;
-        s.init(seed, domain, uint32_t(path_start + p), count);
-        for (uint32_t k = 0; k < count; ++k) {
-            double z = 0.0;
-            const int status = zig_sample(s, zig, &z);
-            if (status != kNormalOk) {
+        NormalStream<kSimulateThreads> s;
+        s.init(normals, domain, uint32_t(path_start + p));
+        for (uint32_t k = 0; k < count; k += kChunkNormals) {
+            double z[kChunkNormals];
+            if (!s.next4(keys, k, count, z)) {
                 atomicMin(fail, (unsigned long long)p);
                 break;
             }
-            out[p * count + k] = z;
+#pragma unroll
+            for (uint32_t j = 0; j < kChunkNormals; ++j)
+                if (k + j < count) out[p * count + k + j] = z[j];
         }
     }
 }
@@ -108,12 +112,12 @@ __global__ void __launch_bounds__(256) normals_kernel(uint64_t seed, uint32_t do
 // K1: seeded simulation with time-major row stores.
 // ---------------------------------------------------------------------------------------------
 
-__global__ void __launch_bounds__(256) simulate_kernel(DevicePlan plan, uint64_t paths, uint64_t seed,
-                                                       uint32_t domain, double* out, uint32_t store_first_row,
-                                                       int reconstruct_escrowed, unsigned long long* fail) {
-    __shared__ double sx[257], sf[257];
-    load_zig_tables(sx, sf);
-    const SmemZig zig = make_zig(sx, sf);
+__global__ void __launch_bounds__(kSimulateThreads, 4) simulate_kernel(DevicePlan plan, uint64_t paths, PhiloxKeys keys,
+                                                                    uint32_t domain, double* out,
+                                                                    uint32_t store_first_row, int reconstruct_escrowed,
+                                                                    unsigned long long* fail) {
+    __shared__ NormalSmem<kSimulateThreads> normals;
+    load_normal_tables(normals);
     for (uint64_t p = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; p < paths;
          p += uint64_t(gridDim.x) * blockDim.x) {
         auto store = [&](int row, double value) {
@@ -124,7 +128,7 @@ __global__ void __launch_bounds__(256) simulate_kernel(DevicePlan plan, uint64_t
             }
             out[uint64_t(row - store_first_row) * paths + p] = value;
         };
-        const SimResult r = simulate_path(plan, zig, seed, domain, uint32_t(p), store);
+        const SimResult r = simulate_path(plan, normals, keys, domain, uint32_t(p), store);
         if (r.code != 0) atomicMin(fail, (unsigned long long)p);
     }
 }
@@ -161,12 +165,12 @@ __global__ void replay_external_kernel(DevicePlan plan, uint64_t paths, const do
 // Re-runs one path serially to recover the typed failure details and the state at `want_row`.
 __global__ void replay_kernel(DevicePlan plan, uint64_t seed, uint32_t domain, uint32_t path, int want_row,
                               SimFailure* out) {
-    __shared__ double sx[257], sf[257];
-    load_zig_tables(sx, sf);
+    __shared__ NormalSmem<kReplayThreads> normals;
+    load_normal_tables(normals);
     if (threadIdx.x != 0) return;
-    const SmemZig zig = make_zig(sx, sf);
+    const PhiloxKeys keys = philox_keys(seed);
     double observed = 0.0;
-    const SimResult r = simulate_path(plan, zig, seed, domain, path, [&](int row, double v) {
+    const SimResult r = simulate_path(plan, normals, keys, domain, path, [&](int row, double v) {
         if (row == want_row) observed = v;
     });
     out->code = r.code;
@@ -184,6 +188,7 @@ struct BackwardSmem {
     double red[32 * kSlots];
     dd total[kSlots];
     FitModel model;
+    ExerciseRule rule;
     double new_pivot;  // the row's own mean, when its sums are taken again about it
     int kind;
     int wait_failed;
@@ -384,6 +389,7 @@ __global__ void __launch_bounds__(kBackwardThreads, 1) backward_kernel(BackwardA
                 fit_continuation_warp(sm.total, fit_pivot, itm, degree, plan.rank_tolerance, plan.rank_limit,
                                       &sm.model);
                 kind = sm.model.status == kFitOk ? kRuleRegression : kRuleFitFailed;
+                if (threadIdx.x == 0 && kind == kRuleRegression) sm.rule = make_exercise_rule(sm.model, D, K);
             }
             if (threadIdx.x == 0) sm.kind = kind;
             if (blockIdx.x == 0 && kind != kRecenterRow) {
@@ -453,7 +459,8 @@ __global__ void __launch_bounds__(kBackwardThreads, 1) backward_kernel(BackwardA
         const int kind = sm.kind;
         if (kind == kRuleFitFailed) return;  // identical decision in every CTA
         const bool regression = kind == kRuleRegression;
-        const FitModel& model = sm.model;  // read from shared memory
+        const ExerciseRule& rule = sm.rule;  // read from shared memory
+        const bool plain = regression && rule.general == 0;
         const double disc = stage_next ? plan.disc_from_later[row - 1] : 1.0;
         const double* cur_row = row_ptr(uint32_t(row));
         const double* next_row = stage_next ? row_ptr(uint32_t(row - 1)) : cur_row;
@@ -465,13 +472,16 @@ __global__ void __launch_bounds__(kBackwardThreads, 1) backward_kernel(BackwardA
             double v = value(j);
             if (regression) {
                 const double sp = kHbm ? __ldcg(&cur_row[p]) : spots[at];
-                if (sp > K) {
-                    const double intrinsic = sp - K;
-                    double continuation;
-                    if (!predict_continuation_d<D>(model, divide(sp, Kd), &continuation)) {
-                        atomicMin(&a.status->fit_predict_fail, ((unsigned long long)order << 32) | p);
-                    } else if (exercise_rule(plan.tie_rule, intrinsic, continuation)) {
-                        v = intrinsic;
+                const double excess = sp - K;
+                if (excess > 0.0) {
+                    if (plain && within_rule(sp)) {
+                        if (exercise_rule(plan.tie_rule, excess, rule_continuation<D>(rule, excess))) v = excess;
+                    } else {
+                        const int decision = decide_general<D>(&sm.model, sp, K, plan.tie_rule);
+                        if (decision == kDecideNonFinite)
+                            atomicMin(&a.status->fit_predict_fail, ((unsigned long long)order << 32) | p);
+                        else if (decision == kDecideExercise)
+                            v = excess;
                     }
                 }
             }
@@ -500,7 +510,7 @@ __global__ void __launch_bounds__(kBackwardThreads, 1) backward_kernel(BackwardA
         spots = spots_next;
         spots_next = swap;
         fit_pivot = stage_pivot;
-        if (regression) latest_mean = model.mean;
+        if (regression) latest_mean = sm.model.mean;
         // Consecutive exchanges use alternate partial buffers: a CTA overwrites a buffer only after
         // every CTA has arrived at the exchange in between, that is, has finished reading it.
         parity ^= 1;
@@ -559,41 +569,24 @@ __global__ void diagnose_kernel(DevicePlan plan, FitRecord* records) {
 // K4: fused re-simulation + fixed-policy evaluation.
 // ---------------------------------------------------------------------------------------------
 
-struct EvalRow {
-    FitModel model;
-    int32_t kind;
-    int32_t pad;
-    double discount;
-};
 
 template <int D>
 __global__ void __launch_bounds__(kEvalThreads, 4) evaluate_kernel(EvalArgs a) {
     extern __shared__ __align__(16) unsigned char eval_smem_raw[];
     const DevicePlan& plan = a.plan;
     const uint32_t rows = plan.rows;
-    double* sx = reinterpret_cast<double*>(eval_smem_raw);
-    double* sf = sx + 257;
-    double* red = sf + 257;                                      // [32 * 2]
-    EvalRow* rules = reinterpret_cast<EvalRow*>(red + 64);       // [rows]
+    __shared__ NormalSmem<kEvalThreads> normals;
+    __shared__ double red[32 * 2];
+    EvalRow* rules = reinterpret_cast<EvalRow*>(eval_smem_raw);      // [rows]
     unsigned* counts = reinterpret_cast<unsigned*>(rules + rows);    // [rows]
     unsigned* itm_counts = counts + rows;                            // [rows]
+    const double K = plan.strike;
     for (uint32_t r = threadIdx.x; r < rows; r += blockDim.x) {
-        EvalRow er;
-        if (r + 1 < rows) {
-            er.model = a.records[r].model;
-            er.kind = a.records[r].kind;
-        } else {
-            er.kind = kRuleNone;
-        }
-        er.discount = plan.disc_to_origin[r];
-        rules[r] = er;
+        rules[r] = make_eval_row(plan, a.records, r);
         counts[r] = 0;
         itm_counts[r] = 0;
     }
-    load_zig_tables(sx, sf);
-    const SmemZig zig = make_zig(sx, sf);
-    const double K = plan.strike;
-    const Divisor Kd = make_divisor(K);
+    load_normal_tables(normals);
     const uint64_t P = plan.eval_paths;
     double sum = 0.0, sumsq = 0.0;
     for (uint64_t p = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; p < P; p += uint64_t(gridDim.x) * blockDim.x) {
@@ -611,19 +604,10 @@ __global__ void __launch_bounds__(kEvalThreads, 4) evaluate_kernel(EvalArgs a) {
                 if (a.stops) a.stops[p] = uint32_t(row);
                 return;
             }
-            if (er.kind == kRuleNoSupport) {
-                if (spot > K) atomicAdd(&itm_counts[row], 1u);
-                return;
-            }
-            if (er.kind != kRuleRegression || !(spot > K)) return;
-            const double intrinsic = spot - K;
-            double continuation;
-            if (!predict_continuation_d<D>(er.model, divide(spot, Kd), &continuation)) {
-                atomicMin(&a.status->eval_fail, ((unsigned long long)row << 33) | (p << 1));
-                return;
-            }
-            if (exercise_rule(plan.tie_rule, intrinsic, continuation)) {
-                payoff = intrinsic * er.discount;
+            const double excess = spot - K;
+            if (!(excess > 0.0)) return;
+            if (decide_row<D>(plan, a.records, a.status, er.rule, uint32_t(row), p, spot, excess, itm_counts)) {
+                payoff = excess * er.discount;
                 if (!fo_isfinite(payoff))
                     atomicMin(&a.status->eval_fail, ((unsigned long long)row << 33) | (p << 1) | 1ull);
                 active = false;
@@ -631,7 +615,7 @@ __global__ void __launch_bounds__(kEvalThreads, 4) evaluate_kernel(EvalArgs a) {
                 if (a.stops) a.stops[p] = uint32_t(row);
             }
         };
-        const SimResult r = simulate_path(plan, zig, plan.eval_seed, plan.eval_domain, uint32_t(p), observe);
+        const SimResult r = simulate_path<false>(plan, normals, a.keys, plan.eval_domain, uint32_t(p), observe);
         if (r.code != 0) atomicMin(&a.status->eval_sim_fail, (unsigned long long)p);
         sum += payoff;
         sumsq += payoff * payoff;
@@ -677,20 +661,20 @@ __global__ void finalize_kernel(const double2* partials, int blocks, uint64_t pa
 
 cudaError_t launch_normals(uint64_t seed, uint32_t domain, uint32_t path_start, uint64_t paths, uint32_t count,
                            double* out, unsigned long long* fail, cudaStream_t stream) {
-    const int threads = 256;
+    const int threads = kSimulateThreads;
     const uint64_t blocks = (paths + threads - 1) / threads;
     normals_kernel<<<unsigned(blocks < 65535 * 16 ? blocks : 65535 * 16), threads, 0, stream>>>(
-        seed, domain, path_start, paths, count, out, fail);
+        philox_keys(seed), domain, path_start, paths, count, out, fail);
     return cudaGetLastError();
 }
 
 cudaError_t launch_simulate(const DevicePlan& plan, uint64_t paths, uint64_t seed, uint32_t domain, double* out,
                             uint32_t store_first_row, int reconstruct_escrowed, unsigned long long* fail,
                             cudaStream_t stream) {
-    const int threads = 256;
+    const int threads = kSimulateThreads;
     uint64_t blocks = (paths + threads - 1) / threads;
     if (blocks > (1u << 20)) blocks = 1u << 20;
-    simulate_kernel<<<unsigned(blocks), threads, 0, stream>>>(plan, paths, seed, domain, out, store_first_row,
+    simulate_kernel<<<unsigned(blocks), threads, 0, stream>>>(plan, paths, philox_keys(seed), domain, out, store_first_row,
                                                                reconstruct_escrowed, fail);
     return cudaGetLastError();
 }
@@ -717,7 +701,7 @@ cudaError_t launch_replay_external(const DevicePlan& plan, uint64_t paths, const
 
 cudaError_t launch_replay(const DevicePlan& plan, uint64_t seed, uint32_t domain, uint32_t path, int want_row,
                           SimFailure* out, cudaStream_t stream) {
-    replay_kernel<<<1, 32, 0, stream>>>(plan, seed, domain, path, want_row, out);
+    replay_kernel<<<1, kReplayThreads, 0, stream>>>(plan, seed, domain, path, want_row, out);
     return cudaGetLastError();
 }
 
@@ -781,12 +765,12 @@ cudaError_t launch_diagnose(const DevicePlan& plan, FitRecord* records, cudaStre
 }
 
 size_t evaluate_smem_bytes(uint32_t rows) {
-    return sizeof(double) * (257 * 2 + 64) + sizeof(EvalRow) * rows + sizeof(unsigned) * 2 * rows;
+    return sizeof(EvalRow) * rows + sizeof(unsigned) * 2 * rows;
 }
 
 template <int D>
 static cudaError_t launch_evaluate_d(const EvalArgs& args, int blocks, size_t smem, cudaStream_t stream) {
-    if (smem > 48 * 1024) {
+    if (smem > kSmallDynamicSmem) {
         cudaError_t e = cudaFuncSetAttribute(evaluate_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
         if (e != cudaSuccess) return e;
     }

@@ -11,6 +11,9 @@ namespace fo {
 
 constexpr int kBackwardThreads = 1024;
 constexpr int kEvalThreads = 256;
+// Dynamic shared memory that fits beside any kernel's static shared memory without opting in to more
+// than 48 KB a CTA.
+constexpr size_t kSmallDynamicSmem = 512;
 
 struct BackwardArgs {
     DevicePlan plan;
@@ -27,6 +30,7 @@ struct BackwardArgs {
 
 struct EvalArgs {
     DevicePlan plan;
+    PhiloxKeys keys;             // of plan.eval_seed
     const FitRecord* records;
     double2* partials;           // [blocks][2]
     unsigned* counts;            // [rows] stopping counts
