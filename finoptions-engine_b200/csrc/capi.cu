@@ -36,7 +36,7 @@ struct PlanLayout {
     size_t sqrt_dt, dt;       // per-interval sqrt(dt) and dt for the adjoint vega
     size_t greek_partials;    // eval_blocks * kGreekSlots double2
     size_t greek_out;         // kGreekSlots doubles (read back)
-    size_t partials;          // backward partials: 2 * blocks * 16 double2
+    size_t partials;          // exchange buffers of the backward pass (at most 2 * blocks * 16 double2)
     size_t eval_partials;     // eval partials: eval_blocks * 2 double2
     size_t out;               // start of the read-back region
     size_t status, result, records, counts, itm_counts, replay;
@@ -329,31 +329,49 @@ Error plan_launch(fo_lsm_call_plan* plan) {
                                 plan->first_stored_row, plan->hp.escrowed ? 1 : 0, &status->train_sim_fail, s),
                 "training simulation launch");
     FO_CUDA_TRY(mark(1), "event");
-    // K2 backward induction
+    // K2 backward induction: every row's moments, then the serial pass
+    MomentArgs mo{};
+    mo.plan = plan->dp;
+    mo.slab = plan->d_slab;
+    mo.partials = reinterpret_cast<double2*>(dev + L.greek_partials);  // the evaluation's, not needed before it
+    mo.records = records;
+    mo.status = status;
+    mo.exchange = reinterpret_cast<double2*>(dev + L.partials);
+    mo.exchange_words = exchange_words(plan->backward_blocks);
+    const uint32_t fitted_rows = plan->hp.rows() - 1 - (plan->hp.origin_row ? 1u : 0u);
+    if (fitted_rows > 0) {
+        const size_t workspace = sizeof(double2) * kGreekSlots * size_t(plan->eval_blocks);
+        FO_CUDA_TRY(launch_moments(mo, moment_blocks(plan->hp.train_paths, fitted_rows, ex->sms, workspace), s), "moments launch");
+    } else {
+        FO_CUDA_TRY(cudaMemsetAsync(mo.exchange, 0, sizeof(double2) * mo.exchange_words, s), "reset");
+    }
     BackwardArgs b{};
     b.plan = plan->dp;
     b.slab = plan->d_slab;
-    b.partials = reinterpret_cast<double2*>(dev + L.partials);
-    b.partial_stride = size_t(plan->backward_blocks) * 16;
+    b.partials = mo.exchange;
     b.records = records;
     b.status = status;
     b.ppt = plan->ppt;
     b.values = plan->backward_hbm
                    ? plan->d_slab + uint64_t(plan->hp.rows() - plan->first_stored_row) * plan->hp.train_paths
                    : nullptr;
-    FO_CUDA_TRY(launch_backward(b, plan->backward_blocks, plan->ppt, s), "backward launch");
-    FO_CUDA_TRY(mark(2), "event");
-    // K3 diagnostics: nothing on the device reads them, so they run on the side stream next to
-    // the evaluation (inline for a stack executor).
-    cudaStream_t ds = ex->side ? ex->side : s;
+    // K3 diagnostics need the moments only, and nothing on the device reads them: they run on the side
+    // stream next to the serial pass (a stack executor runs them inline after it).
     if (ex->side) {
         FO_CUDA_TRY(cudaEventRecord(ex->fork, s), "event");
         FO_CUDA_TRY(cudaStreamWaitEvent(ex->side, ex->fork, 0), "event");
+        if (plan->timing) FO_CUDA_TRY(cudaEventRecord(plan->marks[5], ex->side), "event");
+        FO_CUDA_TRY(launch_diagnose(plan->dp, records, ex->side), "diagnose launch");
+        if (plan->timing) FO_CUDA_TRY(cudaEventRecord(plan->marks[6], ex->side), "event");
+        FO_CUDA_TRY(cudaEventRecord(ex->join, ex->side), "event");
     }
-    if (plan->timing) FO_CUDA_TRY(cudaEventRecord(plan->marks[5], ds), "event");
-    FO_CUDA_TRY(launch_diagnose(plan->dp, records, ds), "diagnose launch");
-    if (plan->timing) FO_CUDA_TRY(cudaEventRecord(plan->marks[6], ds), "event");
-    if (ex->side) FO_CUDA_TRY(cudaEventRecord(ex->join, ex->side), "event");
+    FO_CUDA_TRY(launch_backward(b, plan->backward_blocks, plan->ppt, s), "backward launch");
+    FO_CUDA_TRY(mark(2), "event");
+    if (!ex->side) {
+        if (plan->timing) FO_CUDA_TRY(cudaEventRecord(plan->marks[5], s), "event");
+        FO_CUDA_TRY(launch_diagnose(plan->dp, records, s), "diagnose launch");
+        if (plan->timing) FO_CUDA_TRY(cudaEventRecord(plan->marks[6], s), "event");
+    }
     if (plan->run_eval) {
         EvalArgs a{};
         a.plan = plan->dp;

@@ -50,7 +50,8 @@ struct FitRecord {
     int32_t diag_rank;
     double diag_condition;
     int32_t diag_aux;
-    int32_t pad;
+    int32_t beyond_rule;     // a training spot lies beyond kRuleSpotLimit (single contracts)
+    uint32_t arrived;        // CTAs whose moments of the row are in (single contracts)
 };
 
 // Device status words. Path-addressed failures keep the lowest key with atomicMin so the host
@@ -66,7 +67,7 @@ struct DeviceStatus {
     unsigned long long fit_nonfinite;    // (order << 32) | path: non-finite ITM predictor/response
     unsigned int fit_failed_order;       // first backward order whose fit failed
     unsigned int barrier_timeout;        // zero-initialised: a grid wait timed out
-    unsigned int arrivals;               // zero-initialised: backward CTA partials published so far
+    unsigned int arrivals;               // zero-initialised: what wait_arrivals counts
 };
 constexpr size_t kStatusNoneBytes = 7 * sizeof(unsigned long long) + sizeof(unsigned int);
 

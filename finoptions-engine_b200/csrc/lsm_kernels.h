@@ -9,24 +9,35 @@
 
 namespace fo {
 
-constexpr int kBackwardThreads = 1024;
+constexpr int kBackwardThreads = 512;
 constexpr int kEvalThreads = 256;
 // Dynamic shared memory that fits beside any kernel's static shared memory without opting in to more
 // than 48 KB a CTA.
 constexpr size_t kSmallDynamicSmem = 512;
 
+// The moments of every fitted row, and the backward pass's exchange buffer back at phase 0.
+struct MomentArgs {
+    DevicePlan plan;
+    const double* slab;          // stored training rows [rows - first_stored_row, paths]
+    double2* partials;           // [fitted rows][blocks][16] CTA totals (unused with one block a row)
+    FitRecord* records;          // [rows]; `arrived` starts at zero
+    DeviceStatus* status;
+    double2* exchange;           // BackwardArgs::partials
+    int exchange_words;          // exchange_words(backward blocks)
+};
+
 struct BackwardArgs {
     DevicePlan plan;
     const double* slab;          // stored training rows [rows - first_stored_row, paths]
-    double2* partials;           // [2][16][blocks] double-double CTA partials (ping-pong), slot-major
-    size_t partial_stride;       // doubles2 per ping-pong half
-    FitRecord* records;          // [rows]
+    double2* partials;           // [2][blocks][8] double-double CTA sums, by exchange parity and slot
+    FitRecord* records;          // [rows]: moments_kernel's
     DeviceStatus* status;
     int ppt;                     // paths per thread
     double* values;              // NULL: values and spots on chip (shared memory); else [train paths]
                                  // values in HBM, spots read from the slab (populations beyond the
                                  // on-chip capacity)
 };
+constexpr int exchange_words(int blocks) { return 2 * 8 * blocks; }
 
 struct EvalArgs {
     DevicePlan plan;
@@ -75,6 +86,8 @@ cudaError_t launch_simulate_external(const DevicePlan& plan, uint64_t paths, con
                                      unsigned long long* fail, cudaStream_t stream);
 cudaError_t launch_replay_external(const DevicePlan& plan, uint64_t paths, const double* normals, uint64_t path,
                                    SimFailure* out, cudaStream_t stream);
+int moment_blocks(uint64_t paths, uint32_t rows, int sms, size_t workspace_bytes);
+cudaError_t launch_moments(const MomentArgs& args, int blocks, cudaStream_t stream);
 int backward_max_blocks(int device);
 int backward_max_ppt();
 size_t backward_smem_bytes(int ppt);
