@@ -64,7 +64,7 @@ struct fo_lsm_call_plan {
     DevicePlan dp{};
     bool launched = false;
     // Per-kernel timing marks (created on first timed launch): [0..4] on the plan's stream around
-    // simulate, backward, evaluate and finalize; [5], [6] around the diagnostic on whichever stream
+    // simulate, moments, backward and evaluate; [5], [6] around the diagnostic on whichever stream
     // runs it; [8], [9] bracket a timed series.
     cudaEvent_t marks[10] = {};
     bool timing = false;
@@ -238,6 +238,7 @@ void fill_greeks_args(fo_lsm_call_plan* plan) {
     g.sqrt_dt = reinterpret_cast<const double*>(dev + plan->lay.sqrt_dt);
     g.dt = reinterpret_cast<const double*>(dev + plan->lay.dt);
     g.partials = reinterpret_cast<double2*>(dev + plan->lay.greek_partials);
+    g.sums = reinterpret_cast<double*>(dev + plan->lay.greek_out);
 }
 
 Error plan_create(fo_executor* ex, const fo_lsm_call_request& q, bool own_memory, fo_lsm_call_plan** out) {
@@ -365,8 +366,9 @@ Error plan_launch(fo_lsm_call_plan* plan) {
         if (plan->timing) FO_CUDA_TRY(cudaEventRecord(plan->marks[6], ex->side), "event");
         FO_CUDA_TRY(cudaEventRecord(ex->join, ex->side), "event");
     }
-    FO_CUDA_TRY(launch_backward(b, plan->backward_blocks, plan->ppt, s), "backward launch");
     FO_CUDA_TRY(mark(2), "event");
+    FO_CUDA_TRY(launch_backward(b, plan->backward_blocks, plan->ppt, s), "backward launch");
+    FO_CUDA_TRY(mark(3), "event");
     if (!ex->side) {
         if (plan->timing) FO_CUDA_TRY(cudaEventRecord(plan->marks[5], s), "event");
         FO_CUDA_TRY(launch_diagnose(plan->dp, records, s), "diagnose launch");
@@ -381,15 +383,8 @@ Error plan_launch(fo_lsm_call_plan* plan) {
         a.counts = reinterpret_cast<unsigned*>(dev + L.counts);
         a.itm_counts = reinterpret_cast<unsigned*>(dev + L.itm_counts);
         a.status = status;
+        a.result = reinterpret_cast<double*>(dev + L.result);
         FO_CUDA_TRY(launch_evaluation(plan, a), "evaluation launch");
-        FO_CUDA_TRY(mark(3), "event");
-        FO_CUDA_TRY(launch_finalize(a.partials, plan->eval_blocks, plan->hp.eval_paths,
-                                    reinterpret_cast<double*>(dev + L.result), s),
-                    "finalize launch");
-        if (plan->greeks)
-            FO_CUDA_TRY(launch_finalize_greeks(plan->gk.partials, plan->eval_blocks,
-                                               reinterpret_cast<double*>(dev + L.greek_out), s),
-                        "Greeks finalize launch");
         FO_CUDA_TRY(mark(4), "event");
     }
     if (ex->side) FO_CUDA_TRY(cudaStreamWaitEvent(s, ex->join, 0), "event");
@@ -398,8 +393,8 @@ Error plan_launch(fo_lsm_call_plan* plan) {
     return Error{};
 }
 
-// Timed kernel segments of one launch (the Greeks finalize shares the last segment).
-uint64_t kernels_per_launch(const fo_lsm_call_plan* plan) { return plan->run_eval ? 5 : 3; }
+// Kernels of one launch, each a timed segment.
+uint64_t kernels_per_launch(const fo_lsm_call_plan* plan) { return plan->run_eval ? 5 : 4; }
 
 Error plan_time_launches(fo_lsm_call_plan* plan, uint32_t iterations, double* elapsed_ms, double* kernel_ms,
                          uint64_t capacity) {
@@ -409,11 +404,10 @@ Error plan_time_launches(fo_lsm_call_plan* plan, uint32_t iterations, double* el
     const uint64_t kernels = kernels_per_launch(plan);
     std::vector<double> sums(kernels, 0.0);
     cudaEvent_t begin = plan->marks[8], end = plan->marks[9];
-    // Segments in the order simulate, backward, diagnose, evaluate, finalize. The diagnostic runs
-    // beside the evaluation on the side stream, so the evaluation starts where the backward pass
-    // ends; inline, it starts where the diagnostic ends.
+    // Segments in the order simulate, moments, backward, diagnose, evaluate. The diagnostic runs beside
+    // the backward pass on the side stream; inline, the evaluation starts where it ends.
     const bool side = plan->ex->side != nullptr;
-    const std::pair<int, int> segments[5] = {{0, 1}, {1, 2}, {5, 6}, {side ? 2 : 6, 3}, {3, 4}};
+    const std::pair<int, int> segments[5] = {{0, 1}, {1, 2}, {2, 3}, {5, 6}, {side ? 3 : 6, 4}};
     FO_CUDA_TRY(cudaEventRecord(begin, s), "event");
     double total = 0.0;
     for (uint32_t i = 0; i < iterations; ++i) {
@@ -422,7 +416,7 @@ Error plan_time_launches(fo_lsm_call_plan* plan, uint32_t iterations, double* el
         plan->timing = false;
         if (!e.ok()) return e;
         if (kernel_ms) {
-            FO_CUDA_TRY(cudaEventSynchronize(plan->marks[plan->run_eval ? 4 : 2]), "event");
+            FO_CUDA_TRY(cudaEventSynchronize(plan->marks[plan->run_eval ? 4 : 3]), "event");
             FO_CUDA_TRY(cudaEventSynchronize(plan->marks[6]), "event");
             for (uint64_t k = 0; k < kernels; ++k) {
                 float ms = 0.f;
@@ -740,14 +734,8 @@ Error plan_revalue(fo_lsm_call_plan* plan, const fo_lsm_call_request& q, fo_lsm_
         a.counts = reinterpret_cast<unsigned*>(dev + L.counts);
         a.itm_counts = reinterpret_cast<unsigned*>(dev + L.itm_counts);
         a.status = status;
+        a.result = reinterpret_cast<double*>(dev + L.result);
         FO_CUDA_TRY(launch_evaluation(plan, a), "revaluation launch");
-        FO_CUDA_TRY(launch_finalize(a.partials, plan->eval_blocks, plan->hp.eval_paths,
-                                    reinterpret_cast<double*>(dev + L.result), s),
-                    "finalize launch");
-        if (plan->greeks)
-            FO_CUDA_TRY(launch_finalize_greeks(plan->gk.partials, plan->eval_blocks,
-                                               reinterpret_cast<double*>(dev + L.greek_out), s),
-                        "Greeks finalize launch");
     }
     plan->launched = true;
     return plan_collect(plan, result);
@@ -793,6 +781,7 @@ Error plan_stopping_rows(fo_lsm_call_plan* plan, uint32_t* rows_out, uint64_t ca
     a.itm_counts = reinterpret_cast<unsigned*>(dev + L.itm_counts);
     a.status = status;
     a.stops = static_cast<uint32_t*>(stops.ptr);
+    a.result = reinterpret_cast<double*>(dev + L.result);
     FO_CUDA_TRY(launch_evaluate(a, plan->eval_blocks, s), "stopping-row evaluation launch");
     DeviceStatus st{};
     FO_CUDA_TRY(cudaMemcpyAsync(rows_out, stops.ptr, sizeof(uint32_t) * n, cudaMemcpyDeviceToHost, s), "stops copy");

@@ -834,57 +834,69 @@ FO_HD double fo_hypot(double a, double b) {
 #endif
 }
 
-// Returns DiagnoseStatus; writes rank, condition, and aux (basis degree for non-finite).
-FO_HD_NOINLINE int diagnose_design(const FitModel& model, int degree, double rank_tolerance, double condition_limit,
-                          int* rank_out, double* condition_out, int* aux) {
-    const int columns = degree + 1;
-    double t[kMaxColumns * kMaxColumns];
-    for (int i = 0; i < kMaxColumns * kMaxColumns; ++i) t[i] = 0.0;
-    double previous[kMaxColumns], current[kMaxColumns];
-    for (int i = 0; i < kMaxColumns; ++i) {
+// Returns DiagnoseStatus; writes rank, condition, and aux (basis degree for non-finite). Per degree, with
+// every loop but the sweeps unrolled, so that the matrix stays in registers (57 us for a row of degree 4
+// with it in local memory).
+template <int D>
+FO_HD int diagnose_design_d(const FitModel& model, double rank_tolerance, double condition_limit, int* rank_out,
+                            double* condition_out, int* aux) {
+    constexpr int kColumns = D + 1;
+    double t[kColumns][kColumns];
+    double previous[kColumns], current[kColumns];
+#pragma unroll
+    for (int i = 0; i < kColumns; ++i) {
         previous[i] = 0.0;
-        current[i] = 0.0;
+        current[i] = i == 0 ? 1.0 : 0.0;
+#pragma unroll
+        for (int k = 0; k < kColumns; ++k) t[i][k] = 0.0;
     }
-    current[0] = 1.0;
-    for (int j = 0; j <= degree; ++j) {
+#pragma unroll
+    for (int j = 0; j <= D; ++j) {
         const double inverse_norm = 1.0 / fo_sqrt(model.norm[j]);
         if (!fo_isfinite(inverse_norm)) {
             *aux = j;
             return kDiagNonFinite;
         }
-        for (int k = 0; k <= j; ++k) t[j * kMaxColumns + k] = current[k] * inverse_norm;
-        if (j == degree) break;
-        double next[kMaxColumns];
-        for (int i = 0; i < kMaxColumns; ++i) next[i] = 0.0;
+#pragma unroll
+        for (int k = 0; k <= j; ++k) t[j][k] = current[k] * inverse_norm;
+        if (j == D) break;
+        double next[kColumns];
+#pragma unroll
+        for (int i = 0; i < kColumns; ++i) next[i] = 0.0;
+#pragma unroll
         for (int k = 0; k <= j; ++k) {
             next[k + 1] += current[k];
             next[k] -= model.alpha[j] * current[k];
             next[k] -= model.beta[j] * previous[k];
         }
-        for (int i = 0; i < kMaxColumns; ++i) {
-            if (!fo_isfinite(next[i])) {
-                *aux = j + 1;
-                return kDiagNonFinite;
-            }
+        bool finite = true;
+#pragma unroll
+        for (int i = 0; i < kColumns; ++i) finite = finite && fo_isfinite(next[i]);
+        if (!finite) {
+            *aux = j + 1;
+            return kDiagNonFinite;
         }
-        for (int i = 0; i < kMaxColumns; ++i) {
+#pragma unroll
+        for (int i = 0; i < kColumns; ++i) {
             previous[i] = current[i];
             current[i] = next[i];
         }
     }
     const double tolerance = 16.0 * 2.220446049250313e-16;
     bool converged = false;
-    for (int sweep = 0; sweep < 32; ++sweep) {
+#pragma unroll 1
+    for (int sweep = 0; sweep < 32 && !converged; ++sweep) {
         converged = true;
-        for (int left = 0; left + 1 < columns; ++left) {
-            for (int right = left + 1; right < columns; ++right) {
+#pragma unroll
+        for (int left = 0; left + 1 < kColumns; ++left) {
+#pragma unroll
+            for (int right = left + 1; right < kColumns; ++right) {
                 double ln = 0.0, rn = 0.0, cross = 0.0;
-                for (int row = 0; row < columns; ++row) {
-                    const double lv = t[left * kMaxColumns + row];
-                    const double rv = t[right * kMaxColumns + row];
-                    ln = fo_fma(lv, lv, ln);
-                    rn = fo_fma(rv, rv, rn);
-                    cross = fo_fma(lv, rv, cross);
+#pragma unroll
+                for (int row = 0; row < kColumns; ++row) {
+                    ln = fo_fma(t[left][row], t[left][row], ln);
+                    rn = fo_fma(t[right][row], t[right][row], rn);
+                    cross = fo_fma(t[left][row], t[right][row], cross);
                 }
                 if (!fo_isfinite(ln) || !fo_isfinite(rn) || !fo_isfinite(cross) || ln <= 0.0 || rn <= 0.0) {
                     *aux = right;
@@ -897,54 +909,54 @@ FO_HD_NOINLINE int diagnose_design(const FitModel& model, int degree, double ran
                 if (zeta != 0.0) tangent = (zeta > 0.0 ? 1.0 : -1.0) / (fo_fabs(zeta) + fo_hypot(zeta, 1.0));
                 const double cosine = 1.0 / fo_sqrt(fo_fma(tangent, tangent, 1.0));
                 const double sine = cosine * tangent;
-                for (int row = 0; row < columns; ++row) {
-                    const int li = left * kMaxColumns + row, ri = right * kMaxColumns + row;
-                    const double lv = t[li], rv = t[ri];
-                    t[li] = fo_fma(cosine, lv, -sine * rv);
-                    t[ri] = fo_fma(sine, lv, cosine * rv);
+#pragma unroll
+                for (int row = 0; row < kColumns; ++row) {
+                    const double lv = t[left][row], rv = t[right][row];
+                    t[left][row] = fo_fma(cosine, lv, -sine * rv);
+                    t[right][row] = fo_fma(sine, lv, cosine * rv);
                 }
             }
         }
-        if (converged) break;
     }
     if (!converged) {
-        *aux = columns;
+        *aux = kColumns;
         return kDiagNotConverged;
     }
-    double sv[kMaxColumns];
-    for (int c = 0; c < kMaxColumns; ++c) sv[c] = 0.0;
-    for (int c = 0; c < columns; ++c) {
+    double values[kColumns], largest = 0.0, smallest = 0.0;
+#pragma unroll
+    for (int c = 0; c < kColumns; ++c) {
         double sq = 0.0;
-        for (int row = 0; row < columns; ++row) {
-            const double v = t[c * kMaxColumns + row];
-            sq += v * v;
-        }
-        sv[c] = fo_sqrt(sq);
+#pragma unroll
+        for (int row = 0; row < kColumns; ++row) sq += t[c][row] * t[c][row];
+        values[c] = fo_sqrt(sq);
+        largest = c == 0 || values[c] > largest ? values[c] : largest;
+        smallest = c == 0 || values[c] < smallest ? values[c] : smallest;
     }
-    // descending insertion sort
-    for (int i = 1; i < columns; ++i) {
-        const double v = sv[i];
-        int k = i - 1;
-        while (k >= 0 && sv[k] < v) {
-            sv[k + 1] = sv[k];
-            --k;
-        }
-        sv[k + 1] = v;
-    }
-    const double largest = sv[0];
     const double threshold = rank_tolerance * largest;
     int rank = 0;
-    for (int c = 0; c < columns; ++c) rank += sv[c] > threshold ? 1 : 0;
+#pragma unroll
+    for (int c = 0; c < kColumns; ++c) rank += values[c] > threshold ? 1 : 0;
     *rank_out = rank;
-    if (rank < columns) return kDiagRankDeficient;
-    const double condition = largest / sv[columns - 1];
+    if (rank < kColumns) return kDiagRankDeficient;
+    const double condition = largest / smallest;
     *condition_out = condition;
     if (!fo_isfinite(condition)) {
-        *aux = degree;
+        *aux = D;
         return kDiagNonFinite;
     }
     if (condition > condition_limit) return kDiagConditionExceeded;
     return kDiagOk;
+}
+
+FO_HD_NOINLINE int diagnose_design(const FitModel& model, int degree, double rank_tolerance, double condition_limit,
+                                   int* rank_out, double* condition_out, int* aux) {
+    switch (degree) {
+        case 0: return diagnose_design_d<0>(model, rank_tolerance, condition_limit, rank_out, condition_out, aux);
+        case 1: return diagnose_design_d<1>(model, rank_tolerance, condition_limit, rank_out, condition_out, aux);
+        case 2: return diagnose_design_d<2>(model, rank_tolerance, condition_limit, rank_out, condition_out, aux);
+        case 3: return diagnose_design_d<3>(model, rank_tolerance, condition_limit, rank_out, condition_out, aux);
+        default: return diagnose_design_d<4>(model, rank_tolerance, condition_limit, rank_out, condition_out, aux);
+    }
 }
 
 }  // namespace fo

@@ -34,16 +34,17 @@ struct PersistentLaunch {
     const void* kernel;
     size_t smem;
     int grid;
-    int pad;
+    int threads;
 };
 cudaError_t prepare_batch_persistent(const BatchArgs& a, const BatchQueue& q, int strikes, uint32_t rule_rows,
                                      bool stage, int ctas_per_sm, PersistentLaunch* out);
 cudaError_t enqueue_batch_persistent(const PersistentLaunch& launch, const BatchArgs& a, const BatchQueue& q,
                                      uint32_t rule_rows, bool stage, cudaStream_t stream);
-// The same items as kernels of one kind each (simulation, fits, evaluation), run in stream order:
-// q[k] is phase k's part of the queue, and a fourth kernel writes every problem's summary. Each is
-// launched with enqueue_batch_persistent.
+// The same items as kernels of one kind each, run in stream order: simulation, fits, the fitted rows'
+// rules and diagnostics, evaluation, every problem's summary. q[k] is the queue's part of simulation,
+// fits and evaluation. Each is launched with enqueue_batch_persistent.
+constexpr int kBatchPhaseLaunches = 5;
 cudaError_t prepare_batch_phases(const BatchArgs& a, const BatchQueue (&q)[3], int strikes, uint32_t rule_rows,
-                                 bool stage, PersistentLaunch (&out)[4]);
+                                 bool stage, PersistentLaunch (&out)[kBatchPhaseLaunches]);
 
 }  // namespace fo

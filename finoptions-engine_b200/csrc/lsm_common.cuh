@@ -38,7 +38,8 @@ __device__ __forceinline__ bool gbm_step(double spot, double growth, double* nex
 // growth) after every interval and cash(node, state before, amount) after every cash dividend.
 // Mirrors simulate_one_seeded (seeded.rs:399-459) including the terminal-dividend phase order.
 // kInline: a chunk's four steps are unrolled; otherwise (an observer of hundreds of instructions) they
-// loop, with the growth factors parked in shared memory. Four steps' normals and growth
+// loop, with the growth factors parked in shared memory. C: steps a chunk, 2 for paths of at most two
+// intervals (half the normals and exponentials of a chunk of four would be thrown away). A chunk's normals and growth
 // factors are formed side by side (they do not depend on the state): the four exponentials share
 // the polynomial's constants, which a kernel of this register budget otherwise sets up again for
 // each of them (25 of a step's 62 instructions measured).
@@ -49,7 +50,8 @@ struct IgnoreCash {
     __device__ __forceinline__ void operator()(uint32_t, double, double) const {}
 };
 
-template <bool kInline = true, int T, typename Store, typename Step = IgnoreStep, typename Cash = IgnoreCash>
+template <bool kInline = true, int C = kChunkNormals, int T, typename Store, typename Step = IgnoreStep,
+          typename Cash = IgnoreCash>
 __device__ __forceinline__ SimResult simulate_path(const DevicePlan& plan, NormalSmem<T>& normals,
                                                    const PhiloxKeys& keys, uint32_t domain, uint32_t path,
                                                    Store&& store, Step&& step = Step{}, Cash&& cash = Cash{}) {
@@ -59,21 +61,21 @@ __device__ __forceinline__ SimResult simulate_path(const DevicePlan& plan, Norma
     double spot = plan.sim_start;
     SimResult r{0, 0, 0.0, 0.0};
     if (plan.row_node[0] == 0) store(0, spot);
-    for (uint32_t i = 0; i < intervals; i += kChunkNormals) {
-        double z[kChunkNormals], growth[kChunkNormals];
-        if (!s.next4(keys, i, intervals, z)) {
+    for (uint32_t i = 0; i < intervals; i += C) {
+        double z[C], growth[C];
+        if (!s.template next<C>(keys, i, intervals, z)) {
             r.code = kNormalRejection;
             r.interval = int(i);
             return r;
         }
 #pragma unroll
-        for (uint32_t j = 0; j < kChunkNormals; ++j) {
+        for (uint32_t j = 0; j < C; ++j) {
             const StepCoef c = plan.steps[i + j];  // padded to whole chunks
             growth[j] = fo_exp(fo_fma(c.diffusion, z[j], c.log_drift));
         }
         if constexpr (!kInline) {
 #pragma unroll
-            for (uint32_t j = 0; j < kChunkNormals; ++j) normals.parked[j][threadIdx.x] = growth[j];
+            for (uint32_t j = 0; j < C; ++j) normals.parked[j][threadIdx.x] = growth[j];
         }
         const auto advance = [&](uint32_t j, double factor, double normal) -> bool {
             double next;
@@ -100,12 +102,12 @@ __device__ __forceinline__ SimResult simulate_path(const DevicePlan& plan, Norma
         };
         if constexpr (kInline) {
 #pragma unroll
-            for (uint32_t j = 0; j < kChunkNormals; ++j) {
+            for (uint32_t j = 0; j < C; ++j) {
                 if (j > 0 && i + j >= intervals) return r;
                 if (!advance(j, growth[j], z[j])) return r;
             }
         } else {
-            const uint32_t steps = min(kChunkNormals, intervals - i);
+            const uint32_t steps = min(uint32_t(C), intervals - i);
 #pragma unroll 1
             for (uint32_t j = 0; j < steps; ++j)
                 if (!advance(j, normals.parked[j][threadIdx.x], s.normal(i + j))) return r;
@@ -209,30 +211,38 @@ __device__ __forceinline__ dd shfl_dd_down(dd v, int off) {
     return o;
 }
 
-// Sums partials[b * S + k] over b in a fixed order; warp k handles slot k. Identical in every CTA.
+// Slot `slot` of partials[b * S + slot] summed over b in a fixed order, by one warp; lane 0 has the sum.
+template <int S>
+__device__ __forceinline__ dd sum_slot(const double2* partials, int blocks, int slot) {
+    const int lane = threadIdx.x & 31;
+    // Issue the first eight partials of this lane before adding any, so their L2 latencies overlap; the
+    // additions keep the fixed block order.
+    constexpr int kBatch = 8;
+    double2 v[kBatch];
+#pragma unroll
+    for (int i = 0; i < kBatch; ++i) {
+        const int b = lane + 32 * i;
+        v[i] = b < blocks ? __ldcg(&partials[b * S + slot]) : make_double2(0.0, 0.0);
+    }
+    dd acc = dd_make(0.0);
+#pragma unroll
+    for (int i = 0; i < kBatch; ++i)
+        if (lane + 32 * i < blocks) acc = dd_add(acc, dd{v[i].x, v[i].y});
+    for (int b = lane + 32 * kBatch; b < blocks; b += 32) {
+        const double2 w = __ldcg(&partials[b * S + slot]);
+        acc = dd_add(acc, dd{w.x, w.y});
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) acc = dd_add(acc, shfl_dd_down(acc, off));
+    return acc;
+}
+
+// The first S slots by as many warps of a CTA.
 template <int S>
 __device__ __forceinline__ void grid_combine(const double2* partials, int blocks, dd* out /* smem [S] */) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (warp < S) {
-        // Issue the first eight partials of this lane before adding any, so their L2 latencies
-        // overlap; the additions keep the fixed block order.
-        constexpr int kBatch = 8;
-        double2 v[kBatch];
-#pragma unroll
-        for (int i = 0; i < kBatch; ++i) {
-            const int b = lane + 32 * i;
-            v[i] = b < blocks ? __ldcg(&partials[b * S + warp]) : make_double2(0.0, 0.0);
-        }
-        dd acc = dd_make(0.0);
-#pragma unroll
-        for (int i = 0; i < kBatch; ++i)
-            if (lane + 32 * i < blocks) acc = dd_add(acc, dd{v[i].x, v[i].y});
-        for (int b = lane + 32 * kBatch; b < blocks; b += 32) {
-            const double2 w = __ldcg(&partials[b * S + warp]);
-            acc = dd_add(acc, dd{w.x, w.y});
-        }
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) acc = dd_add(acc, shfl_dd_down(acc, off));
+        const dd acc = sum_slot<S>(partials, blocks, warp);
         if (lane == 0) out[warp] = acc;
     }
     __syncthreads();
@@ -261,8 +271,9 @@ __device__ __forceinline__ bool exercise_rule(int tie_rule, double intrinsic, do
 }
 
 // Whether a spot is below kRuleSpotLimit, by its high word (spots are not negative).
-__device__ __forceinline__ bool within_rule(double spot) { return uint32_t(__double2hiint(spot)) < 0x4c700000u; }
+constexpr uint32_t kRuleLimitHigh = 0x4c700000u;
 static_assert(kRuleSpotLimit == 0x1p200, "high word 0x4c700000");
+__device__ __forceinline__ bool within_rule(double spot) { return uint32_t(__double2hiint(spot)) < kRuleLimitHigh; }
 
 // The decision of an in-the-money spot that the row's ExerciseRule does not cover. No ordinary market
 // gets here, but it stays in line: a call in a path loop costs the loop's registers.
@@ -284,8 +295,7 @@ struct RowSums {
 __device__ __forceinline__ bool finite_nonnegative(double v) { return uint32_t(__double2hiint(v)) < 0x7ff00000u; }
 
 // The sums of one in-the-money path but for its count (acc[0]).
-__device__ __forceinline__ void accumulate_moments(RowSums& r, double x, double y, double pivot) {
-    const double t = x - pivot;
+__device__ __forceinline__ void accumulate_centred(RowSums& r, double t, double y) {
     double pw = t;
     r.acc[kPowerSums] += y;
 #pragma unroll
@@ -296,31 +306,8 @@ __device__ __forceinline__ void accumulate_moments(RowSums& r, double x, double 
     }
 }
 
-__device__ __forceinline__ void accumulate_itm(RowSums& r, double x, double y, double pivot) {
-    r.acc[0] += 1.0;
-    accumulate_moments(r, x, y, pivot);
-}
-
-// The halves of accumulate_itm: count and T_1..T_8 of t = x - pivot (they do not depend on the
-// response), and U_0..U_4 of the response y.
-__device__ __forceinline__ void accumulate_powers(RowSums& r, double t) {
-    r.acc[0] += 1.0;
-    double pw = t;
-#pragma unroll
-    for (int k = 1; k < kPowerSums; ++k) {
-        r.acc[k] += pw;
-        pw *= t;
-    }
-}
-
-__device__ __forceinline__ void accumulate_responses(RowSums& r, double t, double y) {
-    r.acc[kPowerSums] += y;
-    double pw = t;
-#pragma unroll
-    for (int k = 1; k < kResponseSums; ++k) {
-        r.acc[kPowerSums + k] = fo_fma(y, pw, r.acc[kPowerSums + k]);
-        pw *= t;
-    }
+__device__ __forceinline__ void accumulate_moments(RowSums& r, double x, double y, double pivot) {
+    accumulate_centred(r, x - pivot, y);
 }
 
 }  // namespace fo

@@ -28,7 +28,7 @@
 
 namespace fo {
 
-template <int D>  // == plan.degree
+template <int D, int C>  // D == plan.degree
 __global__ void __launch_bounds__(kEvalThreads, 4) evaluate_greeks_kernel(EvalArgs a, GreeksArgs gk) {
     extern __shared__ __align__(16) unsigned char greeks_smem_raw[];
     __shared__ double gred[32 * kGreekSlots];
@@ -87,7 +87,7 @@ __global__ void __launch_bounds__(kEvalThreads, 4) evaluate_greeks_kernel(EvalAr
         const auto cash = [&](uint32_t at, double before, double amount) {
             if (active) adj.cash(at, before, amount);
         };
-        const SimResult r = simulate_path<false>(plan, normals, a.keys, plan.eval_domain, uint32_t(p), observe, step, cash);
+        const SimResult r = simulate_path<false, C>(plan, normals, a.keys, plan.eval_domain, uint32_t(p), observe, step, cash);
         if (r.code != 0) atomicMin(&a.status->eval_sim_fail, (unsigned long long)p);
         // The backward recurrence after the path, where its sums are not live through the path's loop.
         if (!active) {
@@ -110,14 +110,13 @@ __global__ void __launch_bounds__(kEvalThreads, 4) evaluate_greeks_kernel(EvalAr
     cta_reduce_dd<kGreekSlots>(gacc, gred, gtot);
     if (threadIdx.x < kGreekSlots)
         gk.partials[size_t(blockIdx.x) * kGreekSlots + threadIdx.x] = make_double2(gtot[threadIdx.x].hi, gtot[threadIdx.x].lo);
-}
-
-// Sums the Greek partials of every block in a fixed order: warp k handles slot k.
-__global__ void __launch_bounds__(32 * kGreekSlots) finalize_greeks_kernel(const double2* partials, int blocks,
-                                                                             double* out) {
-    __shared__ dd total[kGreekSlots];
-    grid_combine<kGreekSlots>(partials, blocks, total);
-    if (threadIdx.x < kGreekSlots) out[threadIdx.x] = dd_round(total[threadIdx.x]);
+    if (!last_cta(a.status)) return;
+    finalize_price(a.partials, int(gridDim.x), P, a.result);
+    // Every slot's total over the blocks in a fixed order, a warp per slot.
+    for (int slot = threadIdx.x >> 5; slot < kGreekSlots; slot += kEvalThreads / 32) {
+        const dd total = sum_slot<kGreekSlots>(gk.partials, int(gridDim.x), slot);
+        if ((threadIdx.x & 31) == 0) gk.sums[slot] = dd_round(total);
+    }
 }
 
 size_t evaluate_greeks_smem_bytes(uint32_t rows) {
@@ -128,12 +127,13 @@ template <int D>
 static cudaError_t launch_evaluate_greeks_d(const EvalArgs& args, const GreeksArgs& greeks, int blocks,
                                             cudaStream_t stream) {
     const size_t smem = evaluate_greeks_smem_bytes(args.plan.rows);
+    const auto kernel =
+        args.plan.intervals <= 2 ? evaluate_greeks_kernel<D, 2> : evaluate_greeks_kernel<D, kChunkNormals>;
     if (smem > kSmallDynamicSmem) {
-        cudaError_t e =
-            cudaFuncSetAttribute(evaluate_greeks_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
         if (e != cudaSuccess) return e;
     }
-    evaluate_greeks_kernel<D><<<blocks, kEvalThreads, smem, stream>>>(args, greeks);
+    kernel<<<blocks, kEvalThreads, smem, stream>>>(args, greeks);
     return cudaGetLastError();
 }
 
@@ -145,11 +145,6 @@ cudaError_t launch_evaluate_greeks(const EvalArgs& args, const GreeksArgs& greek
         case 3: return launch_evaluate_greeks_d<3>(args, greeks, blocks, stream);
         default: return launch_evaluate_greeks_d<4>(args, greeks, blocks, stream);
     }
-}
-
-cudaError_t launch_finalize_greeks(const double2* partials, int blocks, double* out, cudaStream_t stream) {
-    finalize_greeks_kernel<<<1, 32 * kGreekSlots, 0, stream>>>(partials, blocks, out);
-    return cudaGetLastError();
 }
 
 }  // namespace fo

@@ -1549,8 +1549,9 @@ Error price_groups(fo_executor* ex, const BatchMethod& m, const std::vector<Grou
             }
             cudaEvent_t* mark = ex->batch_marks;
             int grid = 0;
-            PersistentLaunch launch[4] = {};
-            const int n_launches = tune.phases ? 4 : 1;
+            PersistentLaunch launch[kBatchPhaseLaunches] = {};
+            const int n_launches = tune.phases ? kBatchPhaseLaunches : 1;
+            static_assert(kBatchPhaseLaunches <= FO_BATCH_KERNELS, "a timing mark after each launch");
             if (tune.phases) {
                 FO_CUDA_TRY(prepare_batch_phases(a, qs, eval_strikes, max_rows, stage, launch), "batch launch");
                 grid = launch[1].grid;
@@ -1572,7 +1573,7 @@ Error price_groups(fo_executor* ex, const BatchMethod& m, const std::vector<Grou
                 // during capture would only order the captured work).
                 if (ce == cudaSuccess) ce = cudaEventRecordWithFlags(mark[0], s, cudaEventRecordExternal);
                 for (int k = 0; k < n_launches && ce == cudaSuccess; ++k) {
-                    ce = enqueue_batch_persistent(launch[k], a, tune.phases ? qs[k < 3 ? k : 2] : q, max_rows, stage, s);
+                    ce = enqueue_batch_persistent(launch[k], a, tune.phases ? qs[k < 2 ? k : 2] : q, max_rows, stage, s);
                     if (ce == cudaSuccess) ce = cudaEventRecordWithFlags(mark[k + 1], s, cudaEventRecordExternal);
                 }
                 if (ce == cudaSuccess) ce = cudaMemcpyAsync(back, dev + L.out_begin, L.out_bytes, cudaMemcpyDeviceToHost, s);
@@ -1627,9 +1628,11 @@ Error price_groups(fo_executor* ex, const BatchMethod& m, const std::vector<Grou
             FO_CUDA_TRY(cudaStreamSynchronize(s), "batch pricing");
             FO_CUDA_TRY(cudaEventElapsedTime(launch_ms, mark[0], mark[n_launches]), "event");
             for (int k = 0; k < 3; ++k) phase_ms[k] = 0.f;
-            if (tune.phases)  // the summary kernel is counted with the evaluation
+            if (tune.phases) {  // the diagnostics are counted with the fits, the summaries with the evaluation
+                const int from[3] = {0, 1, 3}, to[3] = {1, 3, 5};
                 for (int k = 0; k < 3; ++k)
-                    FO_CUDA_TRY(cudaEventElapsedTime(&phase_ms[k], mark[k], mark[k == 2 ? 4 : k + 1]), "event");
+                    FO_CUDA_TRY(cudaEventElapsedTime(&phase_ms[k], mark[from[k]], mark[to[k]]), "event");
+            }
             if (*timed_out)
                 return make_error(FO_ERR_EXECUTION, FO_CODE_BARRIER_TIMEOUT,
                                   "a batch work item waited too long for the items it depends on; the device result was "

@@ -8,7 +8,7 @@
 //                          (regression.rs:540-577).
 //   K4 evaluate_kernel     re-simulates the evaluation population and applies the fixed policy on
 //                          the fly: no path storage (policy.rs:642-834).
-//   K5 finalize_kernel     price / standard error from the CTA partials (policy.rs:891-926).
+//                          Its last CTA forms price and standard error (policy.rs:891-926).
 //   replay_kernel          re-runs one failing path to recover the typed failure details.
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -23,6 +23,7 @@
 namespace fo {
 
 constexpr int kSimulateThreads = 256;
+constexpr int kSimulateCtasPerSm = 4;
 constexpr int kReplayThreads = 32;
 
 // ---------------------------------------------------------------------------------------------
@@ -41,7 +42,7 @@ __global__ void __launch_bounds__(kSimulateThreads) normals_kernel(PhiloxKeys ke
         s.init(normals, domain, uint32_t(path_start + p));
         for (uint32_t k = 0; k < count; k += kChunkNormals) {
             double z[kChunkNormals];
-            if (!s.next4(keys, k, count, z)) {
+            if (!s.next<kChunkNormals>(keys, k, count, z)) {
                 atomicMin(fail, (unsigned long long)p);
                 break;
             }
@@ -56,7 +57,8 @@ __global__ void __launch_bounds__(kSimulateThreads) normals_kernel(PhiloxKeys ke
 // K1: seeded simulation with time-major row stores.
 // ---------------------------------------------------------------------------------------------
 
-__global__ void __launch_bounds__(kSimulateThreads, 4) simulate_kernel(DevicePlan plan, uint64_t paths, PhiloxKeys keys,
+template <int C>
+__global__ void __launch_bounds__(kSimulateThreads, kSimulateCtasPerSm) simulate_kernel(DevicePlan plan, uint64_t paths, PhiloxKeys keys,
                                                                     uint32_t domain, double* out,
                                                                     uint32_t store_first_row, int reconstruct_escrowed,
                                                                     unsigned long long* fail) {
@@ -72,7 +74,7 @@ __global__ void __launch_bounds__(kSimulateThreads, 4) simulate_kernel(DevicePla
             }
             out[uint64_t(row - store_first_row) * paths + p] = value;
         };
-        const SimResult r = simulate_path(plan, normals, keys, domain, uint32_t(p), store);
+        const SimResult r = simulate_path<true, C>(plan, normals, keys, domain, uint32_t(p), store);
         if (r.code != 0) atomicMin(fail, (unsigned long long)p);
     }
 }
@@ -128,15 +130,17 @@ __global__ void replay_kernel(DevicePlan plan, uint64_t seed, uint32_t domain, u
 // K3: diagnostics for regression rows.
 // ---------------------------------------------------------------------------------------------
 
-__global__ void diagnose_kernel(DevicePlan plan, FitRecord* records) {
-    const uint32_t row = blockIdx.x * blockDim.x + threadIdx.x;
-    if (row + 1 >= plan.rows) return;
+// One row a CTA, by one thread: rows of one warp would wait for each other's rotations and sweeps. Bound by
+// its serial chain of divisions and square roots.
+template <int D>
+__global__ void __launch_bounds__(32) diagnose_kernel(DevicePlan plan, FitRecord* records) {
+    const uint32_t row = blockIdx.x;
     FitRecord& rec = records[row];
-    if (rec.kind != kRuleRegression) return;
+    if (threadIdx.x != 0 || rec.kind != kRuleRegression) return;
     int rank = 0, aux = 0;
     double condition = 0.0;
-    rec.diag_status = diagnose_design(rec.model, plan.degree, plan.rank_tolerance, plan.condition_limit, &rank,
-                                      &condition, &aux);
+    rec.diag_status =
+        diagnose_design_d<D>(rec.model, plan.rank_tolerance, plan.condition_limit, &rank, &condition, &aux);
     rec.diag_rank = rank;
     rec.diag_condition = condition;
     rec.diag_aux = aux;
@@ -147,7 +151,7 @@ __global__ void diagnose_kernel(DevicePlan plan, FitRecord* records) {
 // ---------------------------------------------------------------------------------------------
 
 
-template <int D>
+template <int D, int C>
 __global__ void __launch_bounds__(kEvalThreads, 4) evaluate_kernel(EvalArgs a) {
     extern __shared__ __align__(16) unsigned char eval_smem_raw[];
     const DevicePlan& plan = a.plan;
@@ -192,7 +196,7 @@ __global__ void __launch_bounds__(kEvalThreads, 4) evaluate_kernel(EvalArgs a) {
                 if (a.stops) a.stops[p] = uint32_t(row);
             }
         };
-        const SimResult r = simulate_path<false>(plan, normals, a.keys, plan.eval_domain, uint32_t(p), observe);
+        const SimResult r = simulate_path<false, C>(plan, normals, a.keys, plan.eval_domain, uint32_t(p), observe);
         if (r.code != 0) atomicMin(&a.status->eval_sim_fail, (unsigned long long)p);
         sum += payoff;
         sumsq += payoff * payoff;
@@ -203,33 +207,7 @@ __global__ void __launch_bounds__(kEvalThreads, 4) evaluate_kernel(EvalArgs a) {
         if (counts[r]) atomicAdd(&a.counts[r], counts[r]);
         if (itm_counts[r]) atomicAdd(&a.itm_counts[r], itm_counts[r]);
     }
-}
-
-// ---------------------------------------------------------------------------------------------
-// K5: price and standard error.
-// ---------------------------------------------------------------------------------------------
-
-__global__ void finalize_kernel(const double2* partials, int blocks, uint64_t paths, double* out) {
-    __shared__ dd total[2];
-    grid_combine<2>(partials, blocks, total);
-    if (threadIdx.x == 0) {
-        const dd n = dd_make(double(paths));
-        const dd mean = dd_div(total[0], n);
-        // M2 = sum x^2 - (sum x)^2 / n
-        dd m2 = dd_sub(total[1], dd_mul(total[0], mean));
-        if (m2.hi < 0.0) m2 = dd_make(0.0);
-        out[0] = dd_round(mean);
-        out[1] = dd_round(m2);
-        if (paths > 1) {
-            const dd var = dd_div(m2, dd_make(double(paths - 1)));
-            const double sd = dd_round(dd_sqrt(var));
-            out[2] = sd;
-            out[3] = sd / sqrt(double(paths));
-        } else {
-            out[2] = 0.0;
-            out[3] = 0.0;
-        }
-    }
+    if (last_cta(a.status)) finalize_price(a.partials, int(gridDim.x), P, a.result);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -250,9 +228,15 @@ cudaError_t launch_simulate(const DevicePlan& plan, uint64_t paths, uint64_t see
                             cudaStream_t stream) {
     const int threads = kSimulateThreads;
     uint64_t blocks = (paths + threads - 1) / threads;
+    // A CTA fills 15 KB of sampler tables first, about the work of eight steps: short paths share a CTA's
+    // tables among several blocks of paths, down to one wave of CTAs.
+    const uint64_t share = std::max<uint64_t>(1, 32 / std::max<uint32_t>(plan.intervals, 1));
+    const uint64_t wave = kSimulateCtasPerSm * 148;
+    if (blocks > wave) blocks = std::max<uint64_t>(wave, (blocks + share - 1) / share);
     if (blocks > (1u << 20)) blocks = 1u << 20;
-    simulate_kernel<<<unsigned(blocks), threads, 0, stream>>>(plan, paths, philox_keys(seed), domain, out, store_first_row,
-                                                               reconstruct_escrowed, fail);
+    const auto kernel = plan.intervals <= 2 ? simulate_kernel<2> : simulate_kernel<kChunkNormals>;
+    kernel<<<unsigned(blocks), threads, 0, stream>>>(plan, paths, philox_keys(seed), domain, out, store_first_row,
+                                                     reconstruct_escrowed, fail);
     return cudaGetLastError();
 }
 
@@ -283,8 +267,15 @@ cudaError_t launch_replay(const DevicePlan& plan, uint64_t seed, uint32_t domain
 }
 
 cudaError_t launch_diagnose(const DevicePlan& plan, FitRecord* records, cudaStream_t stream) {
-    const unsigned rows = plan.rows;
-    diagnose_kernel<<<(rows + 63) / 64, 64, 0, stream>>>(plan, records);
+    if (plan.rows <= 1) return cudaSuccess;
+    const unsigned rows = plan.rows - 1;
+    switch (plan.degree) {  // validated to 0..4 on the host
+        case 0: diagnose_kernel<0><<<rows, 32, 0, stream>>>(plan, records); break;
+        case 1: diagnose_kernel<1><<<rows, 32, 0, stream>>>(plan, records); break;
+        case 2: diagnose_kernel<2><<<rows, 32, 0, stream>>>(plan, records); break;
+        case 3: diagnose_kernel<3><<<rows, 32, 0, stream>>>(plan, records); break;
+        default: diagnose_kernel<4><<<rows, 32, 0, stream>>>(plan, records); break;
+    }
     return cudaGetLastError();
 }
 
@@ -294,11 +285,12 @@ size_t evaluate_smem_bytes(uint32_t rows) {
 
 template <int D>
 static cudaError_t launch_evaluate_d(const EvalArgs& args, int blocks, size_t smem, cudaStream_t stream) {
+    const auto kernel = args.plan.intervals <= 2 ? evaluate_kernel<D, 2> : evaluate_kernel<D, kChunkNormals>;
     if (smem > kSmallDynamicSmem) {
-        cudaError_t e = cudaFuncSetAttribute(evaluate_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
         if (e != cudaSuccess) return e;
     }
-    evaluate_kernel<D><<<blocks, kEvalThreads, smem, stream>>>(args);
+    kernel<<<blocks, kEvalThreads, smem, stream>>>(args);
     return cudaGetLastError();
 }
 
@@ -311,11 +303,6 @@ cudaError_t launch_evaluate(const EvalArgs& args, int blocks, cudaStream_t strea
         case 3: return launch_evaluate_d<3>(args, blocks, smem, stream);
         default: return launch_evaluate_d<4>(args, blocks, smem, stream);
     }
-}
-
-cudaError_t launch_finalize(const double2* partials, int blocks, uint64_t paths, double* out, cudaStream_t stream) {
-    finalize_kernel<<<1, 64, 0, stream>>>(partials, blocks, paths, out);
-    return cudaGetLastError();
 }
 
 }  // namespace fo

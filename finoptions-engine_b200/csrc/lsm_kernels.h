@@ -48,6 +48,7 @@ struct EvalArgs {
     unsigned* itm_counts;        // [rows] active in-the-money paths at unsupported rows
     DeviceStatus* status;
     uint32_t* stops;             // optional [evaluation paths]: the row at which each path stopped
+    double* result;              // price, second moment, standard deviation, standard error
 };
 
 // Pathwise adjoint Greeks of the fused evaluation (lsm_greeks.cu).
@@ -70,6 +71,7 @@ struct GreeksArgs {
     const double* sqrt_dt;                      // [intervals]
     const double* dt;                           // [intervals]
     double2* partials;                          // [blocks][kGreekSlots] double-double block sums
+    double* sums;                               // [kGreekSlots]: their totals
 };
 
 cudaError_t launch_normals(uint64_t seed, uint32_t domain, uint32_t path_start, uint64_t paths, uint32_t count,
@@ -95,9 +97,7 @@ cudaError_t launch_backward(const BackwardArgs& args, int blocks, int ppt, cudaS
 cudaError_t launch_diagnose(const DevicePlan& plan, FitRecord* records, cudaStream_t stream);
 size_t evaluate_smem_bytes(uint32_t rows);
 cudaError_t launch_evaluate(const EvalArgs& args, int blocks, cudaStream_t stream);
-cudaError_t launch_finalize(const double2* partials, int blocks, uint64_t paths, double* out, cudaStream_t stream);
 size_t evaluate_greeks_smem_bytes(uint32_t rows);
 cudaError_t launch_evaluate_greeks(const EvalArgs& args, const GreeksArgs& greeks, int blocks, cudaStream_t stream);
-cudaError_t launch_finalize_greeks(const double2* partials, int blocks, double* out, cudaStream_t stream);
 
 }  // namespace fo

@@ -26,27 +26,20 @@
 
 namespace fo {
 
-static __constant__ uint64_t c_zig_x[257] = FO_ZIG_NORM_X_BITS;
-static __constant__ uint64_t c_zig_f[257] = FO_ZIG_NORM_F_BITS;
+// In global memory: a warp reads 32 consecutive entries (constant memory serves one a cycle).
+static __device__ const uint64_t g_zig_x[257] = FO_ZIG_NORM_X_BITS;
+static __device__ const uint64_t g_zig_f[257] = FO_ZIG_NORM_F_BITS;
+static __device__ const uint64_t g_zig_wedge[256][4] = FO_ZIG_WEDGE_BITS;
 
 constexpr uint32_t kRing = 8;            // normals a thread holds
 constexpr uint32_t kChunkNormals = kChunkSteps;  // normals taken together: two blocks
 constexpr uint32_t kReserveNormals = 8;  // paths of more normals than this start four words ahead
 
 // A layer's wedge between its edges a < b, with t the position from a to b and h(t) the density's
-// position from f(a) to f(b): |h(t) - (t + bend t (1 - t))| <= gap. The parabola meets h at both ends
-// and in the middle, so its error is at most max|f'''| / 6 * w^3 / (12 sqrt 3) over the density's drop
-// (w = b - a), with |f'''| = |3 x - x^3| f <= (3 b + b^3) f(a). The margin covers the rounding of both
-// sides (under 1e-12: the drop is at least 1.3e-3, the width 4e-3).
+// position from f(a) to f(b): |h(t) - (t + bend t (1 - t))| <= gap (gen_zignor_tables.py).
 struct alignas(16) Wedge {
     double inverse_width, bend, gap, pad;
 };
-
-__device__ __forceinline__ Wedge make_wedge(double a, double b, double fa, double fb) {
-    const double w = b - a, middle = 0.5 * (a + b), drop = fa - fb;
-    const double h = (fa - fo_exp(-0.5 * middle * middle)) / drop;
-    return Wedge{1.0 / w, 4.0 * (h - 0.5), w * w * w * (3.0 * b + b * b * b) * fa / drop * 0.00802 + 1e-10, 0.0};
-}
 
 // Shared memory of a CTA of T sampling threads.
 template <int T>
@@ -61,18 +54,16 @@ struct NormalSmem {
 template <int T>
 __device__ __forceinline__ void load_normal_tables(NormalSmem<T>& sm) {
     for (int i = threadIdx.x; i < 257; i += blockDim.x) {
-        const double fi = bits_to_double(c_zig_f[i]);
-        sm.f[i] = fi;
-        if (i < 256) {
-            const double b = bits_to_double(c_zig_x[i]), a = bits_to_double(c_zig_x[i + 1]);
-            sm.edge[i] = make_double2(b, a);
-            sm.wedge[i] = make_wedge(a, b, bits_to_double(c_zig_f[i + 1]), fi);
-        }
+        sm.f[i] = bits_to_double(g_zig_f[i]);
+        if (i == 256) break;
+        sm.edge[i] = make_double2(bits_to_double(g_zig_x[i]), bits_to_double(g_zig_x[i + 1]));
+        sm.wedge[i] = Wedge{bits_to_double(g_zig_wedge[i][0]), bits_to_double(g_zig_wedge[i][1]),
+                            bits_to_double(g_zig_wedge[i][2]), 0.0};
     }
     __syncthreads();
 }
 
-// One path's stream. The caller takes its normals in chunks of four, in order, with next4.
+// One path's stream. The caller takes its normals in chunks of four, in order, with next.
 // Invariant between chunks: at most four normals wait in the ring. Everything is in line and there is one
 // copy of it: a call in the path loop, even one never taken, costs the caller's registers.
 template <int T>
@@ -98,12 +89,13 @@ struct NormalStream {
         blocks = 0;
     }
 
-    // Normals k .. k + 3 of a path of n (k a multiple of four; those past n are undefined). False
-    // when the sampler gave up on one of them.
-    __device__ __forceinline__ bool next4(const PhiloxKeys& keys, uint32_t k, uint32_t n, double (&z)[4]) {
+    // Normals k .. k + C - 1 of a path of n (k a multiple of C; those past n are undefined). False when the
+    // sampler gave up on one of them. C is kChunkNormals, or 2 for paths of at most two normals.
+    template <int C>
+    __device__ __forceinline__ bool next(const PhiloxKeys& keys, uint32_t k, uint32_t n, double (&z)[C]) {
         const uint32_t left = n - k;
-        const uint32_t want = left < kChunkNormals ? left : kChunkNormals;
-        // Four words a round: one round, two at the start of a path that keeps a reserve, and more for
+        const uint32_t want = left < C ? left : C;
+        // C words a round: one round, two at the start of a path that keeps a reserve, and more for
         // the lanes still short of the chunk (k normals have left the ring). The ring has room: at
         // most four normals wait when a chunk starts, fewer than four in a lane that is short. The
         // reference gives up on a normal after 2^20 rejections (random/normal.rs:66); here the
@@ -111,26 +103,27 @@ struct NormalStream {
         int rounds = k == 0 && n > kReserveNormals ? -1 : 0;
         do {
             if (rounds >= kMaxRejectionIterations) return false;
-            run(keys);
+            run<C / 2>(keys);
             rounds += 1;
         } while (rounds <= 0 || tail - k < want);
 #pragma unroll
-        for (uint32_t j = 0; j < kChunkNormals; ++j) z[j] = ring[((k + j) % kRing) * T];
+        for (uint32_t j = 0; j < C; ++j) z[j] = ring[((k + j) % kRing) * T];
         return true;
     }
     // Normal k of the chunk that next4 handed out last.
     __device__ __forceinline__ double normal(uint32_t k) const { return ring[(k % kRing) * T]; }
 
-    // Two blocks through the sampler.
+    // N blocks through the sampler.
+    template <int N>
     __device__ __forceinline__ void run(const PhiloxKeys& keys) {
-        uint64_t words[4];
-        philox_blocks<2>(blocks, path, domain, keys, words);
-        blocks += 2;
+        uint64_t words[2 * N];
+        philox_blocks<N>(blocks, path, domain, keys, words);
+        blocks += N;
         const uint32_t tail0 = tail, state0 = state;
         const uint64_t held0 = held;
         bool hard = state > kWedge;  // the tail, or a wedge test too close for the parabola
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
+        for (int i = 0; i < 2 * N; ++i) {
             const uint32_t layer = uint32_t(words[i]) & 0xffu;
             const double2 edge = tables->edge[layer];
             double value = zig_symmetric_unit(words[i]) * edge.x;
@@ -163,8 +156,9 @@ struct NormalStream {
             state = state0;
             held = held0;
 #pragma unroll 1
-            for (int i = 0; i < 4; ++i) {
-                const uint64_t low = (i & 1) ? words[1] : words[0], high = (i & 1) ? words[3] : words[2];
+            for (int i = 0; i < 2 * N; ++i) {
+                const uint64_t low = (i & 1) ? words[1] : words[0];
+                const uint64_t high = (i & 1) ? words[2 * N - 1] : words[2 * N - 2];
                 word_by_word((i & 2) ? high : low);
             }
         }

@@ -31,13 +31,16 @@ cudaError_t prepare_batch_persistent(const BatchArgs& a, const BatchQueue& q, in
 }
 
 cudaError_t prepare_batch_phases(const BatchArgs& a, const BatchQueue (&q)[3], int strikes, uint32_t rule_rows,
-                                 bool stage, PersistentLaunch (&out)[4]) {
+                                 bool stage, PersistentLaunch (&out)[kBatchPhaseLaunches]) {
     cudaError_t e = prepare_phase(kPhaseSimulate, a, q[0], strikes, rule_rows, stage, 0, &out[0]);
     if (e == cudaSuccess) e = prepare_phase(kPhaseFit, a, q[1], strikes, rule_rows, stage, 0, &out[1]);
-    if (e == cudaSuccess) e = prepare_phase(kPhaseEvaluate, a, q[2], strikes, rule_rows, stage, 0, &out[2]);
+    if (e == cudaSuccess) e = prepare_phase(kPhaseEvaluate, a, q[2], strikes, rule_rows, stage, 0, &out[3]);
+    const void* const diagnose[5] = {batch_diagnose_entry<0>(), batch_diagnose_entry<1>(), batch_diagnose_entry<2>(),
+                                     batch_diagnose_entry<3>(), batch_diagnose_entry<4>()};
+    out[2] = PersistentLaunch{diagnose[a.degree], 0, int(a.n_problems), kDiagnoseThreads};
     const uint32_t warps = kPersistentThreads / 32;
-    out[3] = PersistentLaunch{reinterpret_cast<const void*>(batch_summarize_kernel), 0,
-                              int((a.n_problems + warps - 1) / warps), 0};
+    out[4] = PersistentLaunch{reinterpret_cast<const void*>(batch_summarize_kernel), 0,
+                              int((a.n_problems + warps - 1) / warps), kPersistentThreads};
     return e;
 }
 
@@ -49,7 +52,7 @@ cudaError_t enqueue_batch_persistent(const PersistentLaunch& launch, const Batch
     uint32_t rows = rule_rows;
     int stage_rules = stage ? 1 : 0;
     void* params[4] = {&args, &queue, &rows, &stage_rules};
-    return cudaLaunchKernel(launch.kernel, dim3(unsigned(launch.grid)), dim3(kPersistentThreads), params, launch.smem,
+    return cudaLaunchKernel(launch.kernel, dim3(unsigned(launch.grid)), dim3(unsigned(launch.threads)), params, launch.smem,
                             stream);
 }
 

@@ -36,11 +36,8 @@ namespace {
 
 constexpr int kPersistentThreads = 256;
 using BatchNormals = NormalSmem<kPersistentThreads>;
-constexpr int kPersistentLoads = 2;  // paths a backward thread loads together
-// The fit kernel of the phase executor runs four CTAs per SM (64 registers a thread): a thread loads
-// one path at a time and reads the row's model from shared memory per path. Resident warps hide the
-// latency better there than paths in flight per thread (measured on the grouped batch).
-constexpr int kFitKernelLoads = 1;
+constexpr int kPersistentLoads = 1;  // paths a backward thread of the persistent launch loads together
+constexpr int kFitKernelLoads = 4;     // ... and one of the fit kernel
 // A dependency wait gives up after this long: one problem's fit on one CTA can take seconds for
 // populations of millions of paths, so the limit is well above any fit's duration.
 constexpr unsigned long long kDependencyTimeoutNs = 20000000000ull;
@@ -198,17 +195,9 @@ struct BackwardItemSmem {
     double new_pivot;  // the row's own mean, when its sums are taken again about it
     int kind;
     int recenter;
+    int beyond[2];     // by order parity: a staged spot or value is beyond kRuleSpotLimit, or not a number
 };
 
-// Backward induction of one problem over the group's stored rows with the problem's values in HBM
-// (policy.rs:215-296, 471-601): per row one deterministic reduction of in-the-money power sums and
-// the regression solve by one warp. A problem of up to kTeamPaths paths is one CTA's; a larger one
-// is split over a team of CTAs (this one is member `member` of `members`), each owning a contiguous
-// range of paths, whose CTA sums are exchanged in member order before every decision, so that every
-// member fits the same model; member 0 writes the records. Thread t owns paths lo + t + m * 256
-// (m = 0, 1, ...), loading kPersistentLoads of them together (kFitKernelLoads in the fit kernel).
-// The order of a thread's paths, and so every sum, does not depend on that count. False when a team
-// exchange gave up.
 // A stored training state. The persistent launch reads rows that other CTAs of the same launch wrote,
 // so through L2 (the SM's L1 is not coherent with other SMs' writes); the fit kernel of the phase
 // executor runs after the simulation kernel has finished, so its reads may use the read-only path.
@@ -218,10 +207,26 @@ __device__ __forceinline__ double load_slab(const double* p) {
     else return __ldcg(p);
 }
 
-template <int D, bool kReadOnlySlab, bool kTeam>
+// Backward induction of one problem over the group's stored rows (policy.rs:215-296, 471-601): per row
+// one deterministic reduction of in-the-money power sums and the regression solve by one warp. A
+// problem of up to kTeamPaths paths is one CTA's; a larger one is split over a team of CTAs (this one
+// is member `member` of `members`), each owning a contiguous range of paths, whose CTA sums are
+// exchanged in member order before every decision, so that every member fits the same model; member
+// 0 writes the records. Thread t owns paths t + 256 m of the range (round m = 0, 1, ...). The values
+// of the first chip_rounds rounds live in shared memory (`chip`), the others in HBM; neither where a
+// value lives nor how many paths a thread loads together (kU) changes the order of a sum.
+// False when a team exchange gave up.
+//
+// What bounds it: a path-row is 36 FP64 operations (72 cycles a warp and scheduler) beside 24 to 32 bytes
+// of L2 traffic, and between two rows' passes stands a serial part (reduce, decide, fit, rule) of 13,000
+// cycles that only the SM's other CTA can fill. At 4,096 states x 8 strikes x 32,768 paths the fits took
+// 271 ms with four CTAs per SM, one path at a time and every value in HBM, its paths decided in a branch of
+// their own. They take 167 ms so: two CTAs (128 registers a thread; with three or four the pass spills, 197
+// and 274 ms), values on chip where they fit, kU = 4 paths side by side without a branch (kU = 2 179 ms,
+// 3 167 ms) and the next four loaded ahead (170 ms without). A row takes 75,000 cycles, 58,000 the pass.
+template <int D, bool kReadOnlySlab, bool kTeam, int kU>
 __device__ bool backward_item(const BatchArgs& a, uint32_t pi, uint32_t member, uint32_t members, unsigned* timeout,
-                              int* flag, BackwardItemSmem& sm) {
-    constexpr int kL = kReadOnlySlab ? kFitKernelLoads : kPersistentLoads;
+                              int* flag, BackwardItemSmem& sm, double* chip, uint32_t chip_rounds) {
     const BatchProblem pr = a.problems[pi];
     if (pr.skip_fit) return true;
     if (status_failed(&a.group_status[pr.group].train_sim_fail)) return true;
@@ -229,114 +234,114 @@ __device__ bool backward_item(const BatchArgs& a, uint32_t pi, uint32_t member, 
     const DevicePlan plan = g.plan;  // a local copy: its fields stay in registers (no reloads across stores)
     ProblemStatus* st = a.problem_status + pi;
     FitRecord* records = a.records + pr.records;
-    // Restrict-qualified: this problem's values are its own, and the slab is only read here, so the
-    // loads of several paths may be issued together, ahead of the stores.
-    double* __restrict__ values = a.values + pr.values;
-    const double* __restrict__ slab = a.slab + g.slab_offset;
+    constexpr uint32_t T = kPersistentThreads;
     const uint64_t P = plan.train_paths;
-    const unsigned T = blockDim.x;
-    const uint64_t step = uint64_t(T) * kL;
     // This member's paths [lo, hi): contiguous ranges of a multiple of 256 paths, in member order.
     const uint64_t span = members == 1 ? P : ((P + members - 1) / members + 255) / 256 * 256;
     const uint64_t lo = members == 1 ? 0 : (uint64_t(member) * span < P ? uint64_t(member) * span : P);
     const uint64_t hi = members == 1 ? P : (lo + span < P ? lo + span : P);
-    const uint64_t first = lo + threadIdx.x;
+    const uint32_t n = uint32_t(hi - lo);
+    const uint32_t full = n / T, rest = n % T;  // rounds in which every thread has a path, and the last one's paths
+    const uint32_t rounds = full + (threadIdx.x < rest ? 1u : 0u);  // this thread's
+    // Restrict-qualified: this problem's values are its own, and the slab is only read here, so the
+    // loads of several paths may be issued together, ahead of the stores.
+    double* __restrict__ values = a.values + pr.values + lo + threadIdx.x;
+    const double* __restrict__ slab = a.slab + g.slab_offset + lo + threadIdx.x;
+    chip += threadIdx.x;
     Team team{member, members, a.team_slots + pr.team_base, a.team_arrive + pi, 0u, timeout, flag};
     const bool writer = member == 0;
     const double K = pr.strike;
     const Divisor Kd = make_divisor(K);
     const int degree = a.degree;
+    const bool strict = a.tie_rule == 0;
     const uint32_t E = plan.rows - 1;
     const uint32_t fsr = plan.first_stored_row;
     const int lowest = plan.origin_row ? 1 : 0;
     auto row_ptr = [&](uint32_t row) { return slab + uint64_t(row - fsr) * P; };
-    {
-        const double* terminal = row_ptr(E);
-        for (uint64_t base = first; base < hi; base += step) {
-            double s[kL];
-#pragma unroll
-            for (int u = 0; u < kL; ++u) {
-                const uint64_t p = base + uint64_t(u) * T;
-                s[u] = p < hi ? load_slab<kReadOnlySlab>(&terminal[p]) : 0.0;
-            }
-#pragma unroll
-            for (int u = 0; u < kL; ++u) {
-                const uint64_t p = base + uint64_t(u) * T;
-                const double d = s[u] - K;
-                if (p < hi) values[p] = d > 0.0 ? d : 0.0;
-            }
-        }
-    }
-    uint32_t order = 0;
-    int row = int(E) - 1;
-    double pivot = 1.0;
-    RowSums sums;
-    uint32_t itm_paths = 0;  // in-the-money paths in the sums (sums.acc[0], counted in integers)
-#pragma unroll
-    for (int k = 0; k < kSlots; ++k) sums.acc[k] = 0.0;
+    auto load_value = [&](uint32_t m) { return m < chip_rounds ? chip[m * T] : values[m * T]; };
+    auto store_value = [&](uint32_t m, double v) {
+        if (m < chip_rounds) chip[m * T] = v;
+        else values[m * T] = v;
+    };
+    auto key = [&](uint32_t order, uint32_t m) {
+        return ((unsigned long long)order << 32) | (lo + threadIdx.x + uint64_t(m) * T);
+    };
     // Moneyness of an in-the-money state: the correctly rounded quotient by the strike.
     const auto moneyness = [&](double spot) {
         const double x = Kd.inv != 0.0 ? divide_above(spot, Kd) : spot / K;
         return finite_nonnegative(x) ? x : spot / K;
     };
+    if (threadIdx.x < 2) sm.beyond[threadIdx.x] = 0;
+    __syncthreads();
+    uint32_t order = 0;
+    int row = int(E) - 1;
+    double pivot = 1.0;
+    RowSums sums;
+    uint32_t itm_paths = 0;  // in-the-money paths in the sums (sums.acc[0], counted in integers)
+    auto clear_sums = [&] {
+#pragma unroll
+        for (int k = 0; k < kSlots; ++k) sums.acc[k] = 0.0;
+        itm_paths = 0;
+    };
+    // The sums of a row whose discounted values are stored, path by path with every check.
+    auto sum_row = [&](int at, bool report) {
+        clear_sums();
+        const double* spots = row_ptr(uint32_t(at));
+        for (uint32_t m = 0; m < rounds; ++m) {
+            const double v = load_value(m), sp = load_slab<kReadOnlySlab>(&spots[m * T]);
+            const bool finite = fo_isfinite(v);
+            if (report && !finite) atomicMin(&st->fit_payoff_fail, key(order, m));
+            if (!(sp > K)) continue;
+            const double x = moneyness(sp);
+            if (!within_rule(sp)) sm.beyond[order & 1] = 1;
+            if (!finite_nonnegative(x) || !finite) {
+                sums.acc[kBadSlot] += 1.0;
+                if (report) atomicMin(&st->fit_nonfinite, key(order, m));
+            } else {
+                itm_paths += 1;
+                accumulate_moments(sums, x, v, pivot);
+            }
+        }
+    };
+    clear_sums();
+    {
+        // The terminal payoffs, discounted into the first fitted row where there is one.
+        const double* terminal = row_ptr(E);
+        const double disc = row >= lowest ? plan.disc_from_later[row] : 1.0;
+#pragma unroll 4
+        for (uint32_t m = 0; m < rounds; ++m) {
+            const double d = load_slab<kReadOnlySlab>(&terminal[m * T]) - K;
+            store_value(m, (d > 0.0 ? d : 0.0) * disc);
+        }
+    }
     if (row >= lowest) {
-        // Discount into the first fitted row and locate its in-the-money mean (the moment pivot).
-        const double disc = plan.disc_from_later[row];
+        // The in-the-money mean of the first fitted row is its moment pivot.
         const double* srow = row_ptr(uint32_t(row));
         double loc[2] = {0.0, 0.0};
-        for (uint64_t base = first; base < hi; base += step) {
-            double v[kL], s[kL];
-#pragma unroll
-            for (int u = 0; u < kL; ++u) {
-                const uint64_t p = base + uint64_t(u) * T;
-                v[u] = p < hi ? values[p] : 0.0;
-                s[u] = p < hi ? load_slab<kReadOnlySlab>(&srow[p]) : 0.0;
-            }
-#pragma unroll
-            for (int u = 0; u < kL; ++u) {
-                const uint64_t p = base + uint64_t(u) * T;
-                if (p >= hi) continue;
-                v[u] *= disc;
-                values[p] = v[u];
-                if (!fo_isfinite(v[u])) atomicMin(&st->fit_payoff_fail, ((unsigned long long)order << 32) | p);
-                if (s[u] > K) {
-                    const double x = divide(s[u], Kd);
-                    if (fo_isfinite(x)) {
-                        loc[0] += 1.0;
-                        loc[1] += x;
-                    }
-                }
+#pragma unroll 4
+        for (uint32_t m = 0; m < rounds; ++m) {
+            const double sp = load_slab<kReadOnlySlab>(&srow[m * T]);
+            if (!(sp > K)) continue;
+            const double x = moneyness(sp);
+            if (fo_isfinite(x)) {
+                loc[0] += 1.0;
+                loc[1] += x;
             }
         }
         cta_reduce_dd<2>(loc, sm.red, sm.total);
         if (!team_exchange<2, kTeam>(team, sm.total)) return false;
         if (sm.total[0].hi > 0.0) pivot = dd_round(dd_div(sm.total[1], sm.total[0]));
-        for (uint64_t base = first; base < hi; base += step) {
-            double v[kL], s[kL];
-#pragma unroll
-            for (int u = 0; u < kL; ++u) {
-                const uint64_t p = base + uint64_t(u) * T;
-                v[u] = p < hi ? values[p] : 0.0;
-                s[u] = p < hi ? load_slab<kReadOnlySlab>(&srow[p]) : 0.0;
-            }
-#pragma unroll
-            for (int u = 0; u < kL; ++u) {
-                const uint64_t p = base + uint64_t(u) * T;
-                if (p >= hi || !(s[u] > K)) continue;
-                const double x = moneyness(s[u]);
-                if (!finite_nonnegative(x) || !finite_nonnegative(v[u])) {
-                    sums.acc[kBadSlot] += 1.0;
-                    atomicMin(&st->fit_nonfinite, ((unsigned long long)order << 32) | p);
-                } else {
-                    itm_paths += 1;
-                    accumulate_moments(sums, x, v[u], pivot);
-                }
-            }
-        }
+        sum_row(row, true);
     }
     for (; row >= lowest; --row, ++order) {
         sums.acc[0] = double(itm_paths);
         cta_reduce_dd<kSlots>(sums.acc, sm.red, sm.total);
+        if (sm.beyond[order & 1] != 0 && order > 0) {
+            // The pass that staged the row formed its sums without looking at what lies beyond the limit.
+            sum_row(row, true);
+            sums.acc[0] = double(itm_paths);
+            cta_reduce_dd<kSlots>(sums.acc, sm.red, sm.total);
+        }
         if (!team_exchange<kSlots, kTeam>(team, sm.total)) return false;
         if (threadIdx.x == 0) {
             const uint64_t itm = uint64_t(sm.total[0].hi);
@@ -350,28 +355,10 @@ __device__ bool backward_item(const BatchArgs& a, uint32_t pi, uint32_t member, 
         __syncthreads();
         if (sm.recenter) {
             // The pivot lay more than a standard deviation from the row's in-the-money mean: take
-            // the row's sums again about that mean (values[] holds the row's discounted values).
+            // the row's sums again about that mean.
             pivot = sm.new_pivot;
-            const double* cur = row_ptr(uint32_t(row));
-#pragma unroll
-            for (int k = 0; k < kSlots; ++k) sums.acc[k] = 0.0;
-            for (uint64_t base = first; base < hi; base += step) {
-                double v[kL], s[kL];
-#pragma unroll
-                for (int u = 0; u < kL; ++u) {
-                    const uint64_t p = base + uint64_t(u) * T;
-                    v[u] = p < hi ? values[p] : 0.0;
-                    s[u] = p < hi ? load_slab<kReadOnlySlab>(&cur[p]) : 0.0;
-                }
-#pragma unroll
-                for (int u = 0; u < kL; ++u) {
-                    const uint64_t p = base + uint64_t(u) * T;
-                    if (p >= hi || !(s[u] > K)) continue;
-                    const double x = divide(s[u], Kd);
-                    if (!fo_isfinite(x) || !fo_isfinite(v[u])) sums.acc[kBadSlot] += 1.0;
-                    else accumulate_itm(sums, x, v[u], pivot);
-                }
-            }
+            sum_row(row, false);
+            sums.acc[0] = double(itm_paths);
             cta_reduce_dd<kSlots>(sums.acc, sm.red, sm.total);
             if (!team_exchange<kSlots, kTeam>(team, sm.total)) return false;
         }
@@ -392,7 +379,6 @@ __device__ bool backward_item(const BatchArgs& a, uint32_t pi, uint32_t member, 
             } else {
                 fit_continuation_warp(sm.total, pivot, itm, degree, a.rank_tolerance, plan.rank_limit, &sm.model);
                 kind = sm.model.status == kFitOk ? kRuleRegression : kRuleFitFailed;
-                if (threadIdx.x == 0 && kind == kRuleRegression) sm.rule = make_exercise_rule(sm.model, D, K);
             }
             FitRecord& rec = records[row];
             constexpr int kModelWords = int(sizeof(FitModel) / sizeof(double2));
@@ -400,7 +386,11 @@ __device__ bool backward_item(const BatchArgs& a, uint32_t pi, uint32_t member, 
             if (writer && threadIdx.x < kModelWords)
                 reinterpret_cast<double2*>(&rec.model)[threadIdx.x] =
                     reinterpret_cast<const double2*>(&sm.model)[threadIdx.x];
-            if (threadIdx.x == 0) sm.kind = kind;
+            if (threadIdx.x == 0) {
+                sm.rule = kind == kRuleRegression ? make_exercise_rule(sm.model, D, K) : never_exercise();
+                sm.kind = kind;
+                sm.beyond[(order + 1) & 1] = 0;
+            }
             if (writer && threadIdx.x == 0) {
                 rec.kind = kind;
                 rec.itm = population;
@@ -413,102 +403,140 @@ __device__ bool backward_item(const BatchArgs& a, uint32_t pi, uint32_t member, 
         __syncthreads();
         const int kind = sm.kind;
         if (kind == kRuleFitFailed) return true;  // the problem's fit raised; the host reports it
-        const bool regression = kind == kRuleRegression;
-        if (regression) pivot = sm.model.mean;
-        // Read at every path instead of held in registers, which go to resident CTAs instead.
-        const volatile ExerciseRule& rule = sm.rule;
-        const bool plain = regression && rule.general == 0;
+        if (kind == kRuleRegression) pivot = sm.model.mean;
         const bool stage_next = row - 1 >= lowest;
+        const bool plain = sm.rule.general == 0 && sm.beyond[order & 1] == 0;
         const double disc = stage_next ? plan.disc_from_later[row - 1] : 1.0;
         const double* cur = row_ptr(uint32_t(row));
         const double* nxt = stage_next ? row_ptr(uint32_t(row - 1)) : cur;
+        clear_sums();
+        if (plain && stage_next && Kd.inv != 0.0) {
+            // The pass proper: decide, discount, add to the next row's sums. Spots and values beyond the
+            // rule's limit are only noticed (their high words' maximum) and looked at after it.
+            const ExerciseRule rule = sm.rule;
+            uint32_t highest = 0;
+            // N paths side by side, without a branch of their own: a path out of the money adds t = 0 and
+            // y = 0, which changes no sum. Groups with none in the money skip the part.
+            const auto group = [&](auto strict_rule, auto& v, auto& sc, auto& sn) {
+                constexpr int N = int(sizeof(v) / sizeof(v[0]));
+                bool decides = false, adds = false;
+                double t[N];
+                bool in[N];
 #pragma unroll
-        for (int k = 0; k < kSlots; ++k) sums.acc[k] = 0.0;
-        itm_paths = 0;
-        // The fit kernel fetches the next step's value and spots before the current step's
-        // arithmetic, so their latency overlaps it (one path per thread and step); the persistent
-        // launch, at two paths per step and the heaviest kind's register budget, fetches in place.
-        constexpr bool kAhead = kReadOnlySlab;
-        double fv[kL], fsc[kL], fsn[kL];
-        auto fetch = [&](uint64_t at) {
+                for (int u = 0; u < N; ++u) {
+                    sc[u] -= K;
+                    decides = decides || sc[u] > 0.0;
+                    in[u] = sn[u] > K;
+                    adds = adds || in[u];
+                }
+                if (decides) {
 #pragma unroll
-            for (int u = 0; u < kL; ++u) {
-                const uint64_t p = at + uint64_t(u) * T;
-                const bool in = p < hi;
-                fv[u] = in ? values[p] : 0.0;
-                fsc[u] = in && regression ? load_slab<kReadOnlySlab>(&cur[p]) : 0.0;
-                fsn[u] = in && stage_next ? load_slab<kReadOnlySlab>(&nxt[p]) : 0.0;
-            }
-        };
-        if constexpr (kAhead) fetch(first);
-        for (uint64_t base = first; base < hi; base += step) {
-            if constexpr (!kAhead) fetch(base);
-            double v[kL], sc[kL], sn[kL];
-#pragma unroll
-            for (int u = 0; u < kL; ++u) {
-                v[u] = fv[u];
-                sc[u] = fsc[u];
-                sn[u] = fsn[u];
-            }
-            if constexpr (kAhead) fetch(base + step);
-#pragma unroll
-            for (int u = 0; u < kL; ++u) {
-                const uint64_t p = base + uint64_t(u) * T;
-                if (p >= hi) continue;
-                const double excess = sc[u] - K;
-                if (regression && excess > 0.0) {
-                    if (plain && within_rule(sc[u])) {
-                        if (exercise_rule(a.tie_rule, excess, rule_continuation<D>(rule, excess))) v[u] = excess;
-                    } else {
-                        const int decision = decide_general<D>(&sm.model, sc[u], K, a.tie_rule);
-                        if (decision == kDecideNonFinite)
-                            atomicMin(&st->fit_predict_fail, ((unsigned long long)order << 32) | p);
-                        else if (decision == kDecideExercise)
-                            v[u] = excess;
+                    for (int u = 0; u < N; ++u) {
+                        const double c = rule_continuation<D>(rule, sc[u]);
+                        v[u] = sc[u] > 0.0 && (decltype(strict_rule)::value ? sc[u] > c : sc[u] >= c) ? sc[u] : v[u];
                     }
                 }
-                if (stage_next) {
+#pragma unroll
+                for (int u = 0; u < N; ++u) {
                     v[u] *= disc;
-                    if (!finite_nonnegative(v[u]))
-                        atomicMin(&st->fit_payoff_fail, ((unsigned long long)(order + 1) << 32) | p);
-                    if (sn[u] > K) {
-                        const double x = moneyness(sn[u]);
-                        if (!finite_nonnegative(x) || !finite_nonnegative(v[u])) {
-                            sums.acc[kBadSlot] += 1.0;
-                            atomicMin(&st->fit_nonfinite, ((unsigned long long)(order + 1) << 32) | p);
-                        } else {
-                            itm_paths += 1;
-                            accumulate_moments(sums, x, v[u], pivot);
+                    highest = max(highest, max(uint32_t(__double2hiint(v[u])), uint32_t(__double2hiint(sn[u]))));
+                }
+                if (adds) {
+                    double y[N];
+#pragma unroll
+                    for (int u = 0; u < N; ++u) {
+                        t[u] = in[u] ? divide_above(sn[u], Kd) - pivot : 0.0;
+                        y[u] = in[u] ? v[u] : 0.0;
+                        itm_paths += in[u] ? 1u : 0u;
+                    }
+#pragma unroll
+                    for (int u = 0; u < N; ++u) accumulate_centred(sums, t[u], y[u]);
+                }
+            };
+            const auto pass = [&](auto strict_rule, auto on_chip, uint32_t from, uint32_t to) {
+                double* const held = decltype(on_chip)::value ? chip : values;
+                uint32_t m = from;
+                if (from + kU <= to) {
+                    // The next kU paths' loads are issued ahead of the current ones' arithmetic; two sets of
+                    // registers take turns.
+                    double v0[kU], c0[kU], n0[kU], v1[kU], c1[kU], n1[kU];
+                    const uint32_t end = to - kU;  // the last whole group's first round
+                    const auto fetch = [&](uint32_t at, auto& v, auto& sc, auto& sn) {
+                        at = min(at, end);
+#pragma unroll
+                        for (int u = 0; u < kU; ++u) {
+                            v[u] = held[(at + u) * T];
+                            sc[u] = load_slab<kReadOnlySlab>(&cur[(at + u) * T]);
+                            sn[u] = load_slab<kReadOnlySlab>(&nxt[(at + u) * T]);
                         }
+                    };
+                    const auto finish = [&](auto& v, auto& sc, auto& sn) {
+                        group(strict_rule, v, sc, sn);
+#pragma unroll
+                        for (int u = 0; u < kU; ++u) held[(m + u) * T] = v[u];
+                        m += kU;
+                    };
+                    fetch(m, v0, c0, n0);
+                    for (;;) {
+                        fetch(m + kU, v1, c1, n1);
+                        finish(v0, c0, n0);
+                        if (m > end) break;
+                        fetch(m + kU, v0, c0, n0);
+                        finish(v1, c1, n1);
+                        if (m > end) break;
                     }
                 }
+                for (; m < to; ++m) {
+                    double v[1] = {held[m * T]}, sc[1] = {load_slab<kReadOnlySlab>(&cur[m * T])},
+                           sn[1] = {load_slab<kReadOnlySlab>(&nxt[m * T])};
+                    group(strict_rule, v, sc, sn);
+                    held[m * T] = v[0];
+                }
+            };
+            const auto run = [&](auto strict_rule) {
+                const uint32_t split = min(chip_rounds, rounds);
+                pass(strict_rule, std::true_type{}, 0, split);
+                pass(strict_rule, std::false_type{}, split, rounds);
+            };
+            if (strict) run(std::true_type{});
+            else run(std::false_type{});
+            if (highest >= kRuleLimitHigh) sm.beyond[(order + 1) & 1] = 1;
+            continue;
+        }
+        // The lowest row, and rows whose spots or rule need the model itself.
+        for (uint32_t m = 0; m < rounds; ++m) {
+            double v = load_value(m);
+            const double sc = load_slab<kReadOnlySlab>(&cur[m * T]);
+            const double excess = sc - K;
+            if (kind == kRuleRegression && excess > 0.0) {
+                if (plain) {
+                    if (exercise_rule(a.tie_rule, excess, rule_continuation<D>(sm.rule, excess))) v = excess;
+                } else {
+                    const int decision = within_rule(sc) && sm.rule.general == 0
+                                             ? (exercise_rule(a.tie_rule, excess, rule_continuation<D>(sm.rule, excess))
+                                                    ? kDecideExercise
+                                                    : kDecideContinue)
+                                             : decide_general<D>(&sm.model, sc, K, a.tie_rule);
+                    if (decision == kDecideNonFinite) atomicMin(&st->fit_predict_fail, key(order, m));
+                    else if (decision == kDecideExercise) v = excess;
+                }
             }
-#pragma unroll
-            for (int u = 0; u < kL; ++u) {
-                const uint64_t p = base + uint64_t(u) * T;
-                if (p < hi) values[p] = v[u];
-            }
+            store_value(m, stage_next ? v * disc : v);
+        }
+        if (stage_next) {
+            order += 1;
+            sum_row(row - 1, true);
+            order -= 1;
         }
     }
     // Common origin decision (policy.rs:265-281): mean of the values discounted to the origin.
     if (plan.origin_row) {
         double acc[2] = {0.0, 0.0};
-        for (uint64_t base = first; base < hi; base += step) {
-            double v[kL];
-#pragma unroll
-            for (int u = 0; u < kL; ++u) {
-                const uint64_t p = base + uint64_t(u) * T;
-                v[u] = p < hi ? values[p] : 0.0;
-            }
-#pragma unroll
-            for (int u = 0; u < kL; ++u) {
-                const uint64_t p = base + uint64_t(u) * T;
-                if (p >= hi) continue;
-                const double w = v[u] * plan.origin_discount;
-                if (!fo_isfinite(w)) atomicMin(&st->fit_payoff_fail, ((unsigned long long)order << 32) | p);
-                acc[0] += 1.0;
-                acc[1] += w;
-            }
+        for (uint32_t m = 0; m < rounds; ++m) {
+            const double w = load_value(m) * plan.origin_discount;
+            if (!fo_isfinite(w)) atomicMin(&st->fit_payoff_fail, key(order, m));
+            acc[0] += 1.0;
+            acc[1] += w;
         }
         cta_reduce_dd<2>(acc, sm.red, sm.total);
         if (!team_exchange<2, kTeam>(team, sm.total)) return false;
@@ -528,7 +556,8 @@ __device__ bool backward_item(const BatchArgs& a, uint32_t pi, uint32_t member, 
 
 // Rank / condition diagnostic of every regression row of problem pi (regression.rs:540-577), and every
 // row's rule for the evaluation; the records were written by this CTA.
-__device__ void diagnose_problem(const BatchArgs& a, uint32_t pi) {
+template <int D>
+__device__ __noinline__ void diagnose_problem(const BatchArgs& a, uint32_t pi) {
     const BatchProblem pr = a.problems[pi];
     const uint32_t rows = a.groups[pr.group].plan.rows;
     for (uint32_t r = threadIdx.x; r + 1 < rows; r += blockDim.x) {
@@ -540,8 +569,8 @@ __device__ void diagnose_problem(const BatchArgs& a, uint32_t pi) {
         if (rec.kind != kRuleRegression) continue;
         int rank = 0, aux = 0;
         double condition = 0.0;
-        rec.diag_status = diagnose_design(rec.model, a.degree, a.rank_tolerance, a.condition_limit, &rank, &condition,
-                                          &aux);
+        rec.diag_status =
+            diagnose_design_d<D>(rec.model, a.rank_tolerance, a.condition_limit, &rank, &condition, &aux);
         rec.diag_rank = rank;
         rec.diag_condition = condition;
         rec.diag_aux = aux;
@@ -991,18 +1020,27 @@ struct PhaseSmem<3, S, true> {
     using type = GreeksItemSmem;
 };
 
+constexpr int kFitCtasPerSm = 2;
+
 template <int kPhase, int S, bool kGreeks>
 struct PhaseOccupancy {
     // Resident CTAs per SM the register budget is cut for.
     static constexpr int value = kPhase == kPhaseSimulate                              ? 4
-                                 : kPhase == kPhaseFit                                   ? 4
+                                 : kPhase == kPhaseFit                                   ? kFitCtasPerSm
                                  : kPhase == kPhaseEvaluate && (S == 1 || kGreeks)       ? 4
                                                                                          : 3;
 };
 
+__device__ __forceinline__ uint32_t dynamic_smem_bytes() {
+    uint32_t bytes;
+    asm("mov.u32 %0, %dynamic_smem_size;" : "=r"(bytes));
+    return bytes;
+}
+
 // S: strikes an evaluation item applies together (kGreeks: one, with the adjoint). The dynamic
 // shared memory holds the staged rules (rule_rows x S ExerciseRules, plus one word per row: whether the row
-// needs its records, or its stopping count with the Greeks) when stage_rules is set.
+// needs its records, or its stopping count with the Greeks) when stage_rules is set; the fit kernel's
+// holds path values.
 template <int kPhase, int S, bool kGreeks, int D>
 __global__ void __launch_bounds__(kPersistentThreads, (PhaseOccupancy<kPhase, S, kGreeks>::value))
     batch_persistent_kernel(BatchArgs a, BatchQueue q, uint32_t rule_rows, int stage_rules) {
@@ -1048,13 +1086,19 @@ __global__ void __launch_bounds__(kPersistentThreads, (PhaseOccupancy<kPhase, S,
                 // The fit kernel runs after the simulation kernel: its dependencies are met.
                 if (kPhase == kPhaseFit || wait_for(&q.sim_done[gi], sim_blocks, q.timeout, &flag)) {
                     // Lone CTAs run a copy of the fit without the team exchanges (fewer live registers).
+                    constexpr bool kOwn = kPhase == kPhaseFit;
+                    constexpr int kU = kOwn ? kFitKernelLoads : kPersistentLoads;
+                    double* const chip = reinterpret_cast<double*>(persistent_dyn);
+                    const uint32_t chip_rounds =
+                        kOwn ? dynamic_smem_bytes() / (kPersistentThreads * uint32_t(sizeof(double))) : 0u;
                     const bool done =
-                        it.count == 1
-                            ? backward_item<D, kPhase == kPhaseFit, false>(a, it.index, 0, 1, q.timeout, &flag, sm.bwd)
-                            : backward_item<D, kPhase == kPhaseFit, true>(a, it.index, it.first, it.count, q.timeout,
-                                                                          &flag, sm.bwd);
+                        it.count == 1 ? backward_item<D, kOwn, false, kU>(a, it.index, 0, 1, q.timeout, &flag, sm.bwd,
+                                                                          chip, chip_rounds)
+                                      : backward_item<D, kOwn, true, kU>(a, it.index, it.first, it.count, q.timeout,
+                                                                         &flag, sm.bwd, chip, chip_rounds);
                     __syncthreads();
-                    if (done && it.first == 0) diagnose_problem(a, it.index);  // member 0 wrote the records
+                    // Member 0 wrote the records; after the fit kernel a kernel of its own diagnoses them.
+                    if (!kOwn && done && it.first == 0) diagnose_problem<D>(a, it.index);
                 }
                 signal_done(&q.bwd_done[gi], 1u);
             }
@@ -1101,7 +1145,15 @@ static cudaError_t prepare_persistent_d(const BatchQueue& q, uint32_t rule_rows,
                                         PersistentLaunch* out) {
     auto kernel = batch_persistent_kernel<kPhase, S, kGreeks, D>;
     const bool rules = stage && (kPhase == kPhaseAll || kPhase == kPhaseEvaluate);
-    const size_t smem = rules ? persistent_rule_bytes(S, kGreeks, rule_rows) : 0;
+    size_t smem = rules ? persistent_rule_bytes(S, kGreeks, rule_rows) : 0;
+    if (kPhase == kPhaseFit) {
+        // What its resident CTAs leave of the SM's shared memory, in whole rounds of path values.
+        cudaFuncAttributes attr{};
+        cudaError_t fe = cudaFuncGetAttributes(&attr, kernel);
+        if (fe != cudaSuccess) return fe;
+        constexpr size_t kSmBytes = 228 * 1024, kReservedPerCta = 1024, kRound = kPersistentThreads * sizeof(double);
+        smem = (kSmBytes / kFitCtasPerSm - kReservedPerCta - attr.sharedSizeBytes) / kRound * kRound;
+    }
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
     if (e != cudaSuccess) return e;
     int per_sm = 0;
@@ -1117,7 +1169,17 @@ static cudaError_t prepare_persistent_d(const BatchQueue& q, uint32_t rule_rows,
     out->kernel = reinterpret_cast<const void*>(kernel);
     out->grid = int(q.n_items) < resident ? int(q.n_items) : resident;
     out->smem = smem;
+    out->threads = kPersistentThreads;
     return cudaSuccess;
+}
+
+// The phase executor's kernel between the fits and the evaluation: every problem's rules and diagnostics, a
+// CTA per problem. In the fit kernel their registers slowed every pass (over 390 ms against 176 at 4,096
+// states x 8 strikes).
+constexpr int kDiagnoseThreads = 64;
+template <int D>
+__global__ void __launch_bounds__(kDiagnoseThreads) batch_diagnose_kernel(BatchArgs a, BatchQueue, uint32_t, int) {
+    if (blockIdx.x < a.n_problems) diagnose_problem<D>(a, blockIdx.x);
 }
 
 // The kernel instances of one degree: the persistent launch (phase kPhaseAll) or one phase's kernel.
@@ -1126,7 +1188,15 @@ template <int D>
 cudaError_t prepare_batch_degree(int phase, bool greeks, int strikes, const BatchQueue& q, uint32_t rule_rows,
                                  bool stage, int ctas_per_sm, PersistentLaunch* out);
 
+template <int D>
+const void* batch_diagnose_entry();
+
 #ifdef FO_BATCH_DEGREE
+template <>
+const void* batch_diagnose_entry<FO_BATCH_DEGREE>() {
+    return reinterpret_cast<const void*>(batch_diagnose_kernel<FO_BATCH_DEGREE>);
+}
+
 template <int kPhase, int D>
 static cudaError_t prepare_phase_degree(bool greeks, int strikes, const BatchQueue& q, uint32_t rule_rows, bool stage,
                                         int ctas_per_sm, PersistentLaunch* out) {
