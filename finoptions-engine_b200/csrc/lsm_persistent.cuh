@@ -132,11 +132,13 @@ __device__ void simulate_item(const BatchArgs& a, uint32_t gi, uint32_t first, u
     for (uint32_t b = first; b < first + count; ++b) {
         const uint64_t p = uint64_t(b) * kPersistentThreads + threadIdx.x;
         if (p >= P) continue;
+        double* at = out + p;  // rows come in order, the unstored origin row first
         auto store = [&](int row, double value) {
             if (uint32_t(row) < fsr) return;
             // Escrowed observations: origin -> S0; otherwise prepaid forward + prepaid cash.
             if (escrowed) value = plan.row_node[row] == 0 ? plan.initial_spot : value + plan.escrow_cash[row];
-            out[uint64_t(row - fsr) * P + p] = value;
+            *at = value;
+            at += P;
         };
         const SimResult r = simulate_path(plan, normals, keys, plan.train_domain, uint32_t(p), store);
         if (r.code != 0) atomicMin(&a.group_status[gi].train_sim_fail, (unsigned long long)p);
@@ -601,10 +603,19 @@ __device__ void cta_reduce_pairs(double (&acc)[2 * S], double* red /* [32 * 2S] 
     __syncthreads();
 }
 
+// A row's rule for one strike, as an evaluation item stages it: the rule's polynomial and the strike in the
+// place of its flag (rows with a flagged rule are decided by the records).
+struct alignas(16) StrikeRule {
+    double slope, shift;
+    double c[kMaxColumns];
+    double strike;
+};
+static_assert(sizeof(StrikeRule) == sizeof(ExerciseRule), "the rules' shared memory is counted in either");
+
 // Shared memory of one evaluation item: S strikes evaluated together by every thread.
 template <int S>
 struct EvalSmem {
-    double red[32 * 2 * S];
+    double red[kPersistentThreads / 32 * 2 * S];
     dd tot[2 * S];
     unsigned cnt[2 * S];
     double strikes[S];
@@ -613,16 +624,20 @@ struct EvalSmem {
     uint32_t problem[S];
 };
 
-// Evaluation blocks [first, first + count) of group gi for strike chunk z: each thread
-// re-simulates one evaluation path per block and applies up to S fitted policies on the fly
-// (policy.rs:642-834); per (problem, block) double-double partials and stopping counts.
-// kStaged: the rules were staged in shared memory, a row's S rules side by side; a row is decided for
-// all S strikes without a branch unless one of them needs its record. Otherwise every row does.
-// Issue-bound: at 4,096 states x 8 strikes x 32,768 paths the phase took 186 ms with the basis
-// recurrence and a branch per strike (1,240 warp instructions a path-step), 92 ms so (486).
+// Evaluation blocks [first, first + count) of group gi for strike chunk z: each thread re-simulates one
+// evaluation path per block and applies up to S fitted policies on the fly (policy.rs:642-834); per
+// (problem, block) double-double partials and stopping counts.
+// kStaged: the rules were staged in shared memory, a row's S rules and strikes side by side; a row is
+// decided for all S strikes without a branch unless one of them needs its record. Otherwise every row does.
+// Issue-bound, its warps too few to hide every latency: at 4,096 states x 8 strikes x 32,768 paths the
+// phase took 186 ms with the basis recurrence and a branch per strike (1,240 warp instructions a
+// path-step), 87 ms with staged rules (486), 72 ms with the strike in the rule, the payoff's sign for the
+// strikes still running and the signs of differences for the comparisons (367), at two CTAs per SM (73.6 at
+// three: their spills leave the little L1 beside 3 x 71 KB of shared memory). With one strike the chunk's
+// steps are unrolled (34.3 -> 31.4 ms for 1,024 ragged contracts); with eight that is slower (78 ms).
 template <int S, int D, bool kStaged, bool kReadOnly>
 __device__ void evaluate_item(const BatchArgs& a, uint32_t gi, uint32_t first, uint32_t count, uint32_t z,
-                              BatchNormals& normals, const PhiloxKeys& keys, EvalSmem<S>& sm, ExerciseRule* staged,
+                              BatchNormals& normals, const PhiloxKeys& keys, EvalSmem<S>& sm, StrikeRule* staged,
                               uint32_t rule_rows) {
     const BatchGroup& g = a.groups[gi];
     const uint32_t p0 = g.first_problem + z * S;
@@ -647,8 +662,13 @@ __device__ void evaluate_item(const BatchArgs& a, uint32_t gi, uint32_t first, u
             const uint32_t k = i / rows, r = i % rows;
             ExerciseRule rule = never_exercise();
             if (int(k) < ns && r + 1 < rows) load_rule<kReadOnly>(&a.rules[sm.rbase[k] + r], &rule);
-            staged[r * S + k] = rule;
             if (rule.general) by_record[r] = 1u;
+            StrikeRule& to = staged[r * S + k];
+            to.slope = rule.slope;
+            to.shift = rule.shift;
+#pragma unroll
+            for (int i = 0; i < kMaxColumns; ++i) to.c[i] = rule.c[i];
+            to.strike = sm.strikes[k];
         }
         __syncthreads();
     }
@@ -658,31 +678,35 @@ __device__ void evaluate_item(const BatchArgs& a, uint32_t gi, uint32_t first, u
         if (threadIdx.x < 2 * S) sm.cnt[threadIdx.x] = 0;
         __syncthreads();
         const uint64_t p = uint64_t(b) * kPersistentThreads + threadIdx.x;
+        // A strike's payoff is -1 until its policy stops the path: its sign is what says that it still runs.
         double payoff[S];
 #pragma unroll
-        for (int k = 0; k < S; ++k) payoff[k] = 0.0;
-        const unsigned all = p < P ? ((1u << ns) - 1u) : 0u;
-        unsigned active = all;  // strikes not exercised yet
+        for (int k = 0; k < S; ++k) payoff[k] = -1.0;
+        const auto running = [&](int k) { return __double2hiint(payoff[k]) < 0; };
+        unsigned expired = 0;  // strikes whose policy reached expiry
         auto observe = [&](int row, double spot) {
-            if (!active) return;
             if (plan.escrowed) spot = plan.row_node[row] == 0 ? plan.initial_spot : spot + plan.escrow_cash[row];
             const double disc = plan.disc_to_origin[row];
             if (uint32_t(row) == last) {
 #pragma unroll
                 for (int k = 0; k < S; ++k) {
-                    if (!((active >> k) & 1u)) continue;
+                    if (k >= ns || !running(k)) continue;
                     const double d = spot - sm.strikes[k];
                     payoff[k] = (d > 0.0 ? d : 0.0) * disc;
+                    expired |= 1u << k;
                     if (!finite_nonnegative(payoff[k]))
                         atomicMin(&a.problem_status[sm.problem[k]].eval_terminal_fail, (unsigned long long)p);
                 }
                 return;
             }
             if (!kStaged || by_record[row] != 0 || !within_rule(spot)) {
+                unsigned open = 0;
+#pragma unroll
+                for (int k = 0; k < S; ++k) open |= running(k) ? 1u << k : 0u;
 #pragma unroll 1
                 for (int k = 0; k < ns; ++k) {
                     const double d = spot - sm.strikes[k];
-                    if (!((active >> k) & 1u) || !(d > 0.0)) continue;
+                    if (!((open >> k) & 1u) || !(d > 0.0)) continue;
                     const int decision = decide_record<D>(a, sm.rbase[k] + row, spot, sm.strikes[k]);
                     ProblemStatus& st = a.problem_status[sm.problem[k]];
                     if (decision == kDecideNonFinite)
@@ -690,37 +714,44 @@ __device__ void evaluate_item(const BatchArgs& a, uint32_t gi, uint32_t first, u
                     if (decision != kDecideExercise) continue;
                     const double paid = d * disc;
                     if (!fo_isfinite(paid)) atomicMin(&st.eval_fail, ((unsigned long long)row << 33) | (p << 1) | 1ull);
-                    active &= ~(1u << k);
 #pragma unroll
-                    for (int m = 0; m < S; ++m) payoff[m] = m == k ? paid : payoff[m];
+                    for (int m = 0; m < S; ++m) payoff[m] = m == k ? fo_fabs(paid) : payoff[m];
                 }
                 return;
             }
-            const ExerciseRule* rules = staged + row * S;
-            const bool strict = a.tie_rule == 0;
+            // Every strike by the signs of K - spot, of the continuation less the excess and of the payoff so
+            // far: a strike without a rule never exercises. (A difference of finite doubles is zero, and
+            // then positive, only where they are equal.)
+            const StrikeRule* rules = staged + row * S;
+            const auto decide = [&](auto strict) {
 #pragma unroll
-            for (int k = 0; k < S; ++k) {
-                const double d = spot - sm.strikes[k];
-                const double c = rule_continuation<D>(rules[k], d);
-                const bool stops = d > 0.0 && (strict ? d > c : d >= c) && ((active >> k) & 1u) != 0;
-                payoff[k] = stops ? d * disc : payoff[k];
-                active = stops ? active & ~(1u << k) : active;
-            }
+                for (int k = 0; k < S; ++k) {
+                    const StrikeRule rule = rules[k];
+                    const double below = rule.strike - spot;
+                    const double c = rule_continuation<D>(rule, -below);
+                    const int kept = decltype(strict)::value ? __double2hiint(c + below) : ~__double2hiint(-below - c);
+                    if ((__double2hiint(below) & kept & __double2hiint(payoff[k])) < 0) payoff[k] = -below * disc;
+                }
+            };
+            if (a.tie_rule == 0) decide(std::true_type{});
+            else decide(std::false_type{});
         };
         if (p < P) {
             const SimResult r =
-                simulate_path<false>(plan, normals, keys, plan.eval_domain, uint32_t(p), observe);
+                simulate_path<(S == 1)>(plan, normals, keys, plan.eval_domain, uint32_t(p), observe);
             if (r.code != 0) atomicMin(&a.group_status[gi].eval_sim_fail, (unsigned long long)p);
         }
         // Paths that stopped early and that reached expiry, per strike.
 #pragma unroll
         for (int k = 0; k < S; ++k) {
-            const unsigned expired = __popc(__ballot_sync(0xffffffffu, (active >> k) & 1u));
-            const unsigned early = __popc(__ballot_sync(0xffffffffu, ((all & ~active) >> k) & 1u));
+            const bool at_expiry = ((expired >> k) & 1u) != 0, stopped = !running(k);
+            const unsigned late = __popc(__ballot_sync(0xffffffffu, at_expiry));
+            const unsigned early = __popc(__ballot_sync(0xffffffffu, stopped && !at_expiry));
             if ((threadIdx.x & 31) == 0) {
                 if (early) atomicAdd(&sm.cnt[2 * k], early);
-                if (expired) atomicAdd(&sm.cnt[2 * k + 1], expired);
+                if (late) atomicAdd(&sm.cnt[2 * k + 1], late);
             }
+            payoff[k] = stopped || at_expiry ? payoff[k] : 0.0;
         }
         double acc[2 * S];
 #pragma unroll
@@ -1024,11 +1055,13 @@ constexpr int kFitCtasPerSm = 2;
 
 template <int kPhase, int S, bool kGreeks>
 struct PhaseOccupancy {
-    // Resident CTAs per SM the register budget is cut for.
-    static constexpr int value = kPhase == kPhaseSimulate                              ? 4
-                                 : kPhase == kPhaseFit                                   ? kFitCtasPerSm
-                                 : kPhase == kPhaseEvaluate && (S == 1 || kGreeks)       ? 4
-                                                                                         : 3;
+    // Resident CTAs per SM the register budget is cut for. The adjoint's at four took 58.1 ms for 1,024
+    // ragged contracts, its state spilled; at three 48.7, at two 52.3.
+    static constexpr int value = kPhase == kPhaseSimulate               ? 4
+                                 : kPhase == kPhaseFit                  ? kFitCtasPerSm
+                                 : kPhase == kPhaseEvaluate && kGreeks  ? 3
+                                 : kPhase == kPhaseEvaluate             ? (S == 1 ? 4 : 2)
+                                                                        : 3;
 };
 
 __device__ __forceinline__ uint32_t dynamic_smem_bytes() {
@@ -1112,11 +1145,12 @@ __global__ void __launch_bounds__(kPersistentThreads, (PhaseOccupancy<kPhase, S,
                                                                       sm.greeks, staged, stops);
                 } else {
                     constexpr bool kRO = kPhase == kPhaseEvaluate;
+                    StrikeRule* rules = reinterpret_cast<StrikeRule*>(persistent_dyn);
                     if (stage_rules)
-                        evaluate_item<S, D, true, kRO>(a, gi, it.first, it.count, it.chunk, normals, keys[1], sm.eval, staged,
+                        evaluate_item<S, D, true, kRO>(a, gi, it.first, it.count, it.chunk, normals, keys[1], sm.eval, rules,
                                                        rule_rows);
                     else
-                        evaluate_item<S, D, false, kRO>(a, gi, it.first, it.count, it.chunk, normals, keys[1], sm.eval, staged,
+                        evaluate_item<S, D, false, kRO>(a, gi, it.first, it.count, it.chunk, normals, keys[1], sm.eval, rules,
                                                         rule_rows);
                 }
             }
