@@ -1056,11 +1056,12 @@ Error evaluation_error(const BatchRun& run, uint64_t g, uint64_t row, const Batc
 
 // ---- orchestration ----------------------------------------------------------------------------------
 
+constexpr size_t kLargestWaveBytes = size_t(48) << 30;
 size_t memory_budget(const fo_executor* ex) {
     size_t free_bytes = 0, total = 0;
     if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess) free_bytes = size_t(8) << 30;
     const size_t usable = size_t(double(free_bytes + ex->batch.bytes) * 0.8);
-    return std::min<size_t>(usable, size_t(48) << 30);
+    return std::min<size_t>(usable, kLargestWaveBytes);
 }
 
 // Request validation in the reference's order (lib.rs:1302-1415, input.rs, pricing.rs:356-400).
@@ -1270,9 +1271,8 @@ Error price_groups(fo_executor* ex, const BatchMethod& m, const std::vector<Grou
     }
 
     // Waves: consecutive groups within the memory budget (and the grid's y extent).
-    const size_t budget = memory_budget(ex);
-    std::vector<Wave> waves;
-    {
+    const auto cut_waves = [&](size_t budget) {
+        std::vector<Wave> waves;
         Wave cur;
         size_t bytes = 0;
         for (uint64_t g = 0; g < launchable; ++g) {
@@ -1309,7 +1309,12 @@ Error price_groups(fo_executor* ex, const BatchMethod& m, const std::vector<Grou
             bytes += cost;
         }
         if (cur.g1 > cur.g0) waves.push_back(cur);
-    }
+        return waves;
+    };
+    // One wave that the arena already holds needs no look at the device's free memory: the query takes the
+    // driver 0.1 to 6 ms (up to 40 seen), against 9 ms of kernels for 128 states x 8 strikes.
+    std::vector<Wave> waves = cut_waves(kLargestWaveBytes);
+    if (waves.size() != 1 || layout_for(waves[0], in_bytes).total > ex->batch.bytes) waves = cut_waves(memory_budget(ex));
     size_t arena = in_bytes;
     for (const Wave& w : waves) arena = std::max(arena, layout_for(w, in_bytes).total);
     Error e = ex->batch.reserve(arena);
