@@ -321,8 +321,7 @@ Error plan_launch(fo_lsm_call_plan* plan) {
     cudaStream_t s = ex->stream;
     auto* status = reinterpret_cast<DeviceStatus*>(dev + L.status);
     auto* records = reinterpret_cast<FitRecord*>(dev + L.records);
-    FO_CUDA_TRY(cudaMemsetAsync(dev + L.out, 0, L.out_bytes, s), "reset");
-    FO_CUDA_TRY(cudaMemsetAsync(status, 0xff, kStatusNoneBytes, s), "reset");
+    FO_CUDA_TRY(launch_reset(dev + L.out, L.out_bytes, status, s), "reset");
     auto mark = [&](int i) -> cudaError_t { return plan->timing ? cudaEventRecord(plan->marks[i], s) : cudaSuccess; };
     FO_CUDA_TRY(mark(0), "event");
     // K1 training simulation
@@ -357,14 +356,23 @@ Error plan_launch(fo_lsm_call_plan* plan) {
                    ? plan->d_slab + uint64_t(plan->hp.rows() - plan->first_stored_row) * plan->hp.train_paths
                    : nullptr;
     // K3 diagnostics need the moments only, and nothing on the device reads them: they run on the side
-    // stream next to the serial pass (a stack executor runs them inline after it).
-    if (ex->side) {
-        FO_CUDA_TRY(cudaEventRecord(ex->fork, s), "event");
+    // stream next to the serial pass (a stack executor runs them inline after it). Where that pass leaves
+    // SMs free, their calls come after the main stream's, which a short contract's kernels would wait for
+    // (two dates, 99 -> 91 us a call); where it takes every SM they would run behind the evaluation's CTAs
+    // (52 weeks, 100,003 paths: 386 us against 372), so they go first.
+    const auto diagnose_aside = [&]() -> Error {
         FO_CUDA_TRY(cudaStreamWaitEvent(ex->side, ex->fork, 0), "event");
         if (plan->timing) FO_CUDA_TRY(cudaEventRecord(plan->marks[5], ex->side), "event");
         FO_CUDA_TRY(launch_diagnose(plan->dp, records, ex->side), "diagnose launch");
         if (plan->timing) FO_CUDA_TRY(cudaEventRecord(plan->marks[6], ex->side), "event");
         FO_CUDA_TRY(cudaEventRecord(ex->join, ex->side), "event");
+        return Error{};
+    };
+    const bool diagnose_first = plan->backward_blocks >= ex->sms;
+    if (ex->side) FO_CUDA_TRY(cudaEventRecord(ex->fork, s), "event");
+    if (ex->side && diagnose_first) {
+        Error e = diagnose_aside();
+        if (!e.ok()) return e;
     }
     FO_CUDA_TRY(mark(2), "event");
     FO_CUDA_TRY(launch_backward(b, plan->backward_blocks, plan->ppt, s), "backward launch");
@@ -386,6 +394,10 @@ Error plan_launch(fo_lsm_call_plan* plan) {
         a.result = reinterpret_cast<double*>(dev + L.result);
         FO_CUDA_TRY(launch_evaluation(plan, a), "evaluation launch");
         FO_CUDA_TRY(mark(4), "event");
+    }
+    if (ex->side && !diagnose_first) {
+        Error e = diagnose_aside();
+        if (!e.ok()) return e;
     }
     if (ex->side) FO_CUDA_TRY(cudaStreamWaitEvent(s, ex->join, 0), "event");
     plan->launched = true;

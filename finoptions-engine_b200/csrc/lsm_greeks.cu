@@ -41,12 +41,14 @@ __global__ void __launch_bounds__(kEvalThreads, 4) evaluate_greeks_kernel(EvalAr
     unsigned* counts = reinterpret_cast<unsigned*>(rules + rows);       // [rows]
     unsigned* itm_counts = counts + rows;                               // [rows]
     const double K = plan.strike;
+    load_normal_tables(normals);
+    await_prior_grid();
     for (uint32_t r = threadIdx.x; r < rows; r += blockDim.x) {
         rules[r] = make_eval_row(plan, a.records, r);
         counts[r] = 0;
         itm_counts[r] = 0;
     }
-    load_normal_tables(normals);
+    __syncthreads();
     const uint64_t P = plan.eval_paths;
     const uint32_t last = rows - 1;
     double sum = 0.0, sumsq = 0.0;
@@ -133,8 +135,7 @@ static cudaError_t launch_evaluate_greeks_d(const EvalArgs& args, const GreeksAr
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
         if (e != cudaSuccess) return e;
     }
-    kernel<<<blocks, kEvalThreads, smem, stream>>>(args, greeks);
-    return cudaGetLastError();
+    return launch_early(kernel, dim3(unsigned(blocks)), kEvalThreads, smem, stream, args, greeks);
 }
 
 cudaError_t launch_evaluate_greeks(const EvalArgs& args, const GreeksArgs& greeks, int blocks, cudaStream_t stream) {

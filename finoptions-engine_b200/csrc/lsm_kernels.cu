@@ -53,6 +53,16 @@ __global__ void __launch_bounds__(kSimulateThreads) normals_kernel(PhiloxKeys ke
     }
 }
 
+// One kernel where two memsets were: each of them took the stream as long.
+__global__ void __launch_bounds__(256) reset_kernel(uint4* region, size_t words, const void* status) {
+    let_next_grid_start();
+    const size_t none = (reinterpret_cast<uintptr_t>(status) - reinterpret_cast<uintptr_t>(region)) / sizeof(uint32_t);
+    static_assert(kStatusNoneBytes % sizeof(uint32_t) == 0, "whole words start as none");
+    const auto word = [&](size_t i) { return i - none < kStatusNoneBytes / sizeof(uint32_t) ? ~0u : 0u; };
+    for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < words; i += size_t(gridDim.x) * blockDim.x)
+        region[i] = make_uint4(word(4 * i), word(4 * i + 1), word(4 * i + 2), word(4 * i + 3));
+}
+
 // ---------------------------------------------------------------------------------------------
 // K1: seeded simulation with time-major row stores.
 // ---------------------------------------------------------------------------------------------
@@ -64,6 +74,7 @@ __global__ void __launch_bounds__(kSimulateThreads, kSimulateCtasPerSm) simulate
                                                                     unsigned long long* fail) {
     __shared__ NormalSmem<kSimulateThreads> normals;
     load_normal_tables(normals);
+    await_prior_grid();
     for (uint64_t p = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; p < paths;
          p += uint64_t(gridDim.x) * blockDim.x) {
         auto store = [&](int row, double value) {
@@ -165,12 +176,14 @@ __global__ void __launch_bounds__(kEvalThreads, 4) evaluate_kernel(EvalArgs a) {
     unsigned* counts = reinterpret_cast<unsigned*>(rules + rows);    // [rows]
     unsigned* itm_counts = counts + rows;                            // [rows]
     const double K = plan.strike;
+    load_normal_tables(normals);
+    await_prior_grid();
     for (uint32_t r = threadIdx.x; r < rows; r += blockDim.x) {
         rules[r] = make_eval_row(plan, a.records, r);
         counts[r] = 0;
         itm_counts[r] = 0;
     }
-    load_normal_tables(normals);
+    __syncthreads();
     const uint64_t P = plan.eval_paths;
     const uint32_t last = rows - 1;
     const uint64_t tie = plan.tie_rule == 0 ? 0u : 1u;
@@ -238,6 +251,13 @@ cudaError_t launch_normals(uint64_t seed, uint32_t domain, uint32_t path_start, 
     return cudaGetLastError();
 }
 
+cudaError_t launch_reset(void* region, size_t bytes, DeviceStatus* status, cudaStream_t stream) {
+    const size_t words = bytes / sizeof(uint4);
+    reset_kernel<<<unsigned(std::min<size_t>((words + 255) / 256, 148)), 256, 0, stream>>>(static_cast<uint4*>(region), words,
+                                                                                          status);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_simulate(const DevicePlan& plan, uint64_t paths, uint64_t seed, uint32_t domain, double* out,
                             uint32_t store_first_row, int reconstruct_escrowed, unsigned long long* fail,
                             cudaStream_t stream) {
@@ -250,9 +270,8 @@ cudaError_t launch_simulate(const DevicePlan& plan, uint64_t paths, uint64_t see
     if (blocks > wave) blocks = std::max<uint64_t>(wave, (blocks + share - 1) / share);
     if (blocks > (1u << 20)) blocks = 1u << 20;
     const auto kernel = plan.intervals <= 2 ? simulate_kernel<2> : simulate_kernel<kChunkNormals>;
-    kernel<<<unsigned(blocks), threads, 0, stream>>>(plan, paths, philox_keys(seed), domain, out, store_first_row,
-                                                     reconstruct_escrowed, fail);
-    return cudaGetLastError();
+    return launch_early(kernel, dim3(unsigned(blocks)), threads, 0, stream, plan, paths, philox_keys(seed), domain, out,
+                        store_first_row, reconstruct_escrowed, fail);
 }
 
 cudaError_t launch_first_nonfinite(const double* values, uint64_t n, unsigned long long* first, cudaStream_t stream) {
@@ -305,8 +324,7 @@ static cudaError_t launch_evaluate_d(const EvalArgs& args, int blocks, size_t sm
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
         if (e != cudaSuccess) return e;
     }
-    kernel<<<blocks, kEvalThreads, smem, stream>>>(args);
-    return cudaGetLastError();
+    return launch_early(kernel, dim3(unsigned(blocks)), kEvalThreads, smem, stream, args);
 }
 
 cudaError_t launch_evaluate(const EvalArgs& args, int blocks, cudaStream_t stream) {
