@@ -398,7 +398,7 @@ def run_ours(args: argparse.Namespace) -> dict | None:
             "d2h_bytes_per_step": int(d2h.value),
             "api": "finoptions.price_lsm_call(executor=CudaExecutor)",
         },
-        "gpu_launches": int(kernels.value) * args.steps,
+        "gpu_launches": (int(kernels.value) + 1) * args.steps,  # the timed kernels and the reset before them
         "roofline": {
             "kernel": dominant,
             # The backward pass is bound by the latency of its 52 dependent row exchanges, not by HBM: achieved / peak below is its
