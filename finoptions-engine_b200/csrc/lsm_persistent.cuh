@@ -586,7 +586,7 @@ __device__ __noinline__ void diagnose_problem(const BatchArgs& a, uint32_t pi) {
 // strike's block totals do not depend on how many strikes an item evaluates together.
 template <int S>
 __device__ void cta_reduce_pairs(double (&acc)[2 * S], double* red /* [32 * 2S] */, dd* out /* [2S] */) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
     for (int k = 0; k < S; ++k) {
         double pair[2] = {acc[2 * k], acc[2 * k + 1]};
@@ -594,12 +594,7 @@ __device__ void cta_reduce_pairs(double (&acc)[2 * S], double* red /* [32 * 2S] 
         if (lane < 2) red[warp * 2 * S + 2 * k + lane] = total;
     }
     __syncthreads();
-    for (int slot = warp; slot < 2 * S; slot += warps) {
-        dd v = dd_make(lane < warps ? red[lane * 2 * S + slot] : 0.0);
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) v = dd_add(v, shfl_dd_down(v, off));
-        if (lane == 0) out[slot] = v;
-    }
+    combine_warps<2 * S>(red, [&](int slot, dd v) { out[slot] = v; });
     __syncthreads();
 }
 
@@ -632,7 +627,7 @@ struct EvalSmem {
 // Issue-bound, its warps too few to hide every latency: at 4,096 states x 8 strikes x 32,768 paths the
 // phase took 186 ms with the basis recurrence and a branch per strike (1,240 warp instructions a
 // path-step), 87 ms with staged rules (486), 72 ms with the strike in the rule, the payoff's sign for the
-// strikes still running and the signs of differences for the comparisons (367), at two CTAs per SM (73.6 at
+// strikes still running and the signs of differences for the comparisons (346), at two CTAs per SM (73.6 at
 // three: their spills leave the little L1 beside 3 x 71 KB of shared memory). With one strike the chunk's
 // steps are unrolled (34.3 -> 31.4 ms for 1,024 ragged contracts); with eight that is slower (78 ms).
 template <int S, int D, bool kStaged, bool kReadOnly>
