@@ -1,7 +1,7 @@
 // The regression solve of one exercise row, run by one warp.
 //
 // fit_near_pivot<D> (fo_core.cuh) holds about 37 doubles live through its recurrence, more than a
-// thread of the 64-register backward kernel has, so a one-thread solve spills on the critical
+// thread of a kernel that keeps paths in registers has, so a one-thread solve spills on the critical
 // path of every row. Here the same solve is spread over the 32 lanes of a converged warp:
 //
 //   * lane k <= 2D shifts power sum k and lane 2D + 1 + k (k <= D) response sum k to moments of
