@@ -16,6 +16,7 @@
 #include "lsm_device.cuh"
 #include "lsm_fit_warp.cuh"
 #include "lsm_kernels.h"
+#include "lsm_row_solve.cuh"
 #include "lsm_sync.cuh"
 
 namespace fo {
@@ -248,87 +249,14 @@ constexpr int kExchangeWarps = 8;
 constexpr int kExchangeLoads = 5;                // CTA lines a lane reads together (148 CTAs: one round)
 constexpr int kFetchThread = (kExchangeWarps + 1) * 32;
 
-// What a fitted row's pass needs of its moments: z = excess * slope + shift, the basis in powers of z
-// and its norms.
-struct RowBasis {
-    double slope, shift;
-    double discount;                         // into this row from the one after it
-    double power[kMaxColumns][kMaxColumns];  // p_j = sum_i power[j][i] z^i
-    double solve[kMaxColumns][kMaxColumns];  // powers' coefficients from the response sums
-    double norm[kMaxColumns], inv_norm[kMaxColumns];
-    double reach[kMaxColumns];               // |z|^i at kRuleSpotLimit
-    double mean, scale, inv_scale;           // rows outside the rule's range
-    int kind;
-    int general;
-};
-
 struct BackwardSmem {
     double red[kBackwardThreads / 32][kExchangeSlots];  // per warp and slot
     dd share[kExchangeWarps][kExchangeSlots];  // the exchange warps' shares of the grid's totals
-    double total[kExchangeSlots];
     RowBasis basis[2];  // of the row being decided and of the row being staged, by row parity
-    ExerciseRule rule;
-    int kind;
+    RowSolution row;    // of the row being decided
     int failed;       // a wait timed out
     uint64_t loaded;  // mbarrier of the staged row's spots
 };
-
-// One warp prepares a row's basis from its record, lane i the coefficient of z^i.
-template <int D>
-__device__ __forceinline__ void prepare_basis(const DevicePlan& plan, const FitRecord* records, int row, RowBasis* out) {
-    const int lane = threadIdx.x & 31;
-    const FitRecord& rec = records[row];
-    const FitModel& m = rec.model;
-    const int kind = rec.kind;
-    const double mean = m.mean, scale = m.scale, strike = plan.strike;
-    const bool fitted = kind == kRuleRegression;
-    const double norm = lane < kMaxColumns ? m.norm[lane] : 0.0;
-    const double inv_norm = make_divisor(norm).inv;
-    double current = lane == 0 ? 1.0 : 0.0, previous = 0.0;
-    double solve[kMaxColumns];
-#pragma unroll
-    for (int k = 0; k < kMaxColumns; ++k) solve[k] = 0.0;
-#pragma unroll
-    for (int j = 0; j <= D; ++j) {
-        if (lane < kMaxColumns) out->power[j][lane] = current;
-        // solve[i][k] = sum_j power[j][i] power[j][k] / norm[j]
-        const double weight = current * __shfl_sync(0xffffffffu, inv_norm, j);
-#pragma unroll
-        for (int k = 0; k <= D; ++k)
-            if (k <= j) solve[k] = fo_fma(weight, __shfl_sync(0xffffffffu, current, k), solve[k]);
-        if (j < D) {
-            const double below = __shfl_up_sync(0xffffffffu, current, 1);
-            const double next =
-                fo_fma(-m.beta[j], previous, fo_fma(-m.alpha[j], current, lane > 0 ? below : 0.0));
-            previous = current;
-            current = next;
-        }
-    }
-    const double slope = D > 0 && fitted ? 1.0 / (strike * scale) : 0.0;
-    const double shift = D > 0 && fitted ? (1.0 - mean) / scale : 0.0;
-    const double z = fo_fma(kRuleSpotLimit, slope, fo_fabs(shift));
-    double reach = 1.0;
-#pragma unroll
-    for (int i = 1; i < kMaxColumns; ++i) reach = i <= lane ? reach * z : reach;
-    if (lane < kMaxColumns) {
-        out->norm[lane] = norm;
-        out->inv_norm[lane] = inv_norm;
-        out->reach[lane] = reach;
-#pragma unroll
-        for (int k = 0; k < kMaxColumns; ++k) out->solve[lane][k] = solve[k];
-    }
-    if (lane == 0) {
-        out->slope = slope;
-        out->shift = shift;
-        out->discount = plan.disc_from_later[row];
-        out->mean = mean;
-        out->scale = scale;
-        out->inv_scale = m.inv_scale;
-        out->kind = kind;
-        out->general = fitted && (rec.beyond_rule != 0 || !(strike > 0x1p-100 && strike < 0x1p100) ||
-                                  !(scale > 0x1p-100 && scale < 0x1p100));
-    }
-}
 
 // Grid-wide sums. A CTA's totals travel as one line of eight 16-byte double-doubles whose lowest bits are
 // the exchange's phase (moving hi's lowest bit into lo costs nothing, lo loses 2^-105 of the sum), so
@@ -437,47 +365,17 @@ __device__ __forceinline__ dd exchange_totals(const BackwardArgs& a, BackwardSme
     return slot_sum(grid);
 }
 
-// A row's rule from its response sums (lane k's `total` is slot k's), by warp 0, lane i the coefficient of
-// z^i: one product with the matrix prepared beside the exchange.
+// The row's coefficients into its record, by one warp of CTA 0; and the failure of a row whose response sums
+// leave no finite coefficient.
 template <int D>
-__device__ __forceinline__ void solve_row(BackwardSmem& sm, const RowBasis& basis, double total) {
+__device__ __forceinline__ void write_coefficients(const RowSolution& row, FitRecord& rec) {
     const int lane = threadIdx.x & 31;
-    const int i = lane <= D ? lane : 0;
-    double c = 0.0;
-#pragma unroll
-    for (int k = 0; k <= D; ++k) c = fo_fma(basis.solve[i][k], __shfl_sync(0xffffffffu, total, k), c);
-    const bool covered = __all_sync(0xffffffffu, fo_fabs(c) * basis.reach[i] < 0x1p1000);
-    const bool finite = covered || __all_sync(0xffffffffu, fo_isfinite(c));
-    const double bad = __shfl_sync(0xffffffffu, total, kBadResponses);
-    if (lane < kExchangeSlots) sm.total[lane] = total;
-    if (lane < kMaxColumns) sm.rule.c[lane] = lane <= D ? c : 0.0;
-    if (lane == 0) {
-        sm.rule.slope = basis.slope;
-        sm.rule.shift = basis.shift;
-        sm.rule.general = basis.general != 0 || !covered;
-        sm.kind = bad > 0.5 || !finite ? kRuleFitFailed : kRuleRegression;
-    }
-}
-
-// The row's coefficients in its orthogonal basis into its record, by one warp of CTA 0, lane j the j-th
-// basis function; and the failure of a row whose response sums leave no finite rule.
-template <int D>
-__device__ __forceinline__ void write_coefficients(const BackwardSmem& sm, const RowBasis& basis, FitRecord& rec) {
-    const int lane = threadIdx.x & 31;
-    const int j = lane <= D ? lane : 0;
-    double projection = 0.0;
-#pragma unroll
-    for (int i = 0; i <= D; ++i)
-        projection = i <= j ? fo_fma(basis.power[j][i], sm.total[i], projection) : projection;
-    const double coef = divide(projection, Divisor{basis.norm[j], basis.inv_norm[j]});
-    if (lane <= D) rec.model.coef[lane] = coef;
-    if (sm.kind == kRuleRegression) return;
-    const unsigned broken = __ballot_sync(0xffffffffu, lane <= D && !(fo_isfinite(projection) && fo_isfinite(coef)));
-    if (lane != 0) return;
+    if (lane <= D) rec.model.coef[lane] = row.coef[lane];
+    if (lane != 0 || row.kind == kRuleRegression) return;
     rec.kind = kRuleFitFailed;
-    if (sm.total[kBadResponses] > 0.5) return;
+    if (row.bad_responses) return;
     rec.model.status = kFitNonFinite;
-    rec.model.aux = broken != 0 ? __ffs(int(broken)) - 1 : 0;
+    rec.model.aux = row.broken;
 }
 
 // A CTA owns ppt * blockDim consecutive paths, a thread every blockDim-th of them. When the population
@@ -533,7 +431,7 @@ __global__ void __launch_bounds__(kBackwardThreads, 1) backward_kernel(BackwardA
     }
     if (threadIdx.x == 0) {
         sm.failed = 0;
-        sm.rule = never_exercise();
+        sm.row.rule = never_exercise();
         mbarrier_init(&sm.loaded, 1);
     }
     double sums[kExchangeSlots];
@@ -571,7 +469,7 @@ __global__ void __launch_bounds__(kBackwardThreads, 1) backward_kernel(BackwardA
     auto pass = [&](int row, int next, uint32_t order) {
         const bool decide = row >= 0, stage = next >= lowest;
         const RowBasis& basis = sm.basis[next & 1];
-        const ExerciseRule& rule = sm.rule;
+        const ExerciseRule& rule = sm.row.rule;
         const double disc = stage ? basis.discount : 1.0;
         const double* cur_row = decide ? row_ptr(row) : nullptr;
         const double* next_row = stage ? row_ptr(next) : nullptr;
@@ -629,21 +527,32 @@ __global__ void __launch_bounds__(kBackwardThreads, 1) backward_kernel(BackwardA
             return;
         }
         // A row outside the rules' range: the same pass through the model itself.
+        struct {
+            double mean, scale, inv_scale, alpha[kMaxDegree], beta[kMaxDegree], coef[kMaxColumns];
+        } model{};
+        if (decide) {
+            const RowBasis& b = sm.basis[row & 1];
+            model.mean = b.mean;
+            model.scale = b.scale;
+            model.inv_scale = b.inv_scale;
+#pragma unroll
+            for (int j = 0; j < D; ++j) {
+                model.alpha[j] = b.alpha[j];
+                model.beta[j] = b.beta[j];
+            }
+#pragma unroll
+            for (int j = 0; j <= D; ++j) model.coef[j] = sm.row.coef[j];
+        }
 #pragma unroll 1
         for (int j = 0; j < owned; ++j) {
             const int at = j * T + threadIdx.x;
             const uint64_t p = first + uint64_t(at);
             double v = value(j);
-            if (decide && sm.kind == kRuleRegression) {
+            if (decide && sm.row.kind == kRuleRegression) {
                 const double sp = kHbm ? __ldcg(&cur_row[at]) : cur_spots[at];
                 if (sp > K) {
-                    const RowBasis& b = sm.basis[row & 1];
-                    const double z =
-                        D == 0 ? 0.0 : divide(divide(sp, Kd) - b.mean, Divisor{b.scale, b.inv_scale});
-                    double continuation = rule.c[D];
-#pragma unroll
-                    for (int k = D - 1; k >= 0; --k) continuation = fo_fma(continuation, z, rule.c[k]);
-                    if (!fo_isfinite(continuation))
+                    double continuation;
+                    if (!predict_continuation_d<D>(model, divide(sp, Kd), &continuation))
                         atomicMin(&a.status->fit_predict_fail, ((unsigned long long)(order - 1) << 32) | p);
                     else if (exercise_rule(plan.tie_rule, sp - K, continuation))
                         v = sp - K;
@@ -680,13 +589,16 @@ __global__ void __launch_bounds__(kBackwardThreads, 1) backward_kernel(BackwardA
         if (lane < kExchangeSlots) sm.red[warp][lane] = total;
         clear_sums();
     };
+    const auto prepare = [&](int at) {
+        prepare_basis<D>(a.records[at], K, plan.disc_from_later[at], &sm.basis[at & 1]);
+    };
     clear_sums();
     unsigned seq = 0;
     uint32_t order = 0;
     int row = int(E) - 1;
     __syncthreads();  // the mbarrier is ready
     if (row >= lowest) {
-        if (warp == kExchangeWarps) prepare_basis<D>(plan, a.records, row, &sm.basis[row & 1]);
+        if (warp == kExchangeWarps) prepare(row);
         if (threadIdx.x == kFetchThread) {
             fetch(row);
             wait_copy();
@@ -710,14 +622,15 @@ __global__ void __launch_bounds__(kBackwardThreads, 1) backward_kernel(BackwardA
         __syncthreads();
         if (warp < kExchangeWarps) {
             if (fits) {
-                const dd total = exchange_totals(a, sm, seq);
-                if (warp == 0) solve_row<D>(sm, basis, dd_round(total));
+                const double total = dd_round(exchange_totals(a, sm, seq));
+                if (warp == 0)
+                    solve_row<D>(basis, total, __shfl_sync(0xffffffffu, total, kBadResponses) > 0.5, &sm.row);
             } else if (threadIdx.x == 0) {
-                sm.rule = never_exercise();
-                sm.kind = kind;
+                sm.row.rule = never_exercise();
+                sm.row.kind = kind;
             }
         } else if (row - 1 >= lowest) {
-            if (warp == kExchangeWarps) prepare_basis<D>(plan, a.records, row - 1, &sm.basis[(row - 1) & 1]);
+            if (warp == kExchangeWarps) prepare(row - 1);
             if (threadIdx.x == kFetchThread) {
                 fetch(row - 1);
                 wait_copy();
@@ -725,8 +638,8 @@ __global__ void __launch_bounds__(kBackwardThreads, 1) backward_kernel(BackwardA
         }
         __syncthreads();
         if (sm.failed) return;
-        if (fits && blockIdx.x == 0 && warp == kExchangeWarps) write_coefficients<D>(sm, basis, a.records[row]);
-        if (sm.kind == kRuleFitFailed) {
+        if (fits && blockIdx.x == 0 && warp == kExchangeWarps) write_coefficients<D>(sm.row, a.records[row]);
+        if (sm.row.kind == kRuleFitFailed) {
             if (blockIdx.x == 0 && threadIdx.x == 0) atomicMin(&a.status->fit_failed_order, order);
             return;
         }
