@@ -99,8 +99,7 @@ __device__ __forceinline__ void load_rule(const ExerciseRule* rule, ExerciseRule
     for (int i = 0; i < 4; ++i) dst[i] = kReadOnly ? __ldg(src + i) : __ldcg(src + i);
 }
 
-// A row that its ExerciseRule does not decide (an unsupported row, an extreme market, or more rules
-// than shared memory holds): the record's kind and, for a regression, its model. An in-the-money
+// A row that its ExerciseRule does not decide (an unsupported row, an extreme market): the record's kind and, for a regression, its model. An in-the-money
 // path at a row without training support is counted.
 template <int D>
 __device__ __forceinline__ int decide_record(const BatchArgs& a, uint32_t record, double spot, double strike) {
@@ -599,7 +598,7 @@ __device__ void cta_reduce_pairs(double (&acc)[2 * S], double* red /* [32 * 2S] 
 }
 
 // A row's rule for one strike, as an evaluation item stages it: the rule's polynomial and the strike in the
-// place of its flag (rows with a flagged rule are decided by the records).
+// place of its flag (a flagged rule is staged as one that never exercises, its strike noted in by_record).
 struct alignas(16) StrikeRule {
     double slope, shift;
     double c[kMaxColumns];
@@ -623,7 +622,9 @@ struct EvalSmem {
 // evaluation path per block and applies up to S fitted policies on the fly (policy.rs:642-834); per
 // (problem, block) double-double partials and stopping counts.
 // kStaged: the rules were staged in shared memory, a row's S rules and strikes side by side; a row is
-// decided for all S strikes without a branch unless one of them needs its record. Otherwise every row does.
+// decided for all S strikes without a branch, and those of them that need their records (an unsupported row,
+// a rule beyond its range) one by one. Otherwise each strike reads its rule from global memory. Either way
+// a strike's decisions are the same arithmetic, whatever strikes are priced beside it.
 // Issue-bound, its warps too few to hide every latency: at 4,096 states x 8 strikes x 32,768 paths the
 // phase took 186 ms with the basis recurrence and a branch per strike (1,240 warp instructions a
 // path-step), 87 ms with staged rules (486), 72 ms with the strike in the rule, the payoff's sign for the
@@ -640,7 +641,7 @@ __device__ void evaluate_item(const BatchArgs& a, uint32_t gi, uint32_t first, u
     if (ns <= 0 || status_failed(&a.group_status[gi].train_sim_fail)) return;  // uniform over the CTA
     const DevicePlan plan = g.plan;  // a local copy: its fields stay in registers (no reloads across stores)
     const uint32_t rows = plan.rows;
-    unsigned* by_record = reinterpret_cast<unsigned*>(staged + size_t(S) * rule_rows);  // [rows], staged rules only
+    unsigned* by_record = reinterpret_cast<unsigned*>(staged + size_t(S) * rule_rows);  // [rows] strikes decided by their records
     if (threadIdx.x < S) {
         const bool live = int(threadIdx.x) < ns;
         const BatchProblem pr = a.problems[live ? p0 + threadIdx.x : p0];
@@ -650,14 +651,17 @@ __device__ void evaluate_item(const BatchArgs& a, uint32_t gi, uint32_t first, u
         sm.problem[threadIdx.x] = live ? p0 + threadIdx.x : p0;
     }
     if constexpr (kStaged)
-        for (uint32_t r = threadIdx.x; r < rows; r += blockDim.x) by_record[r] = plan.disc_to_origin[r] < 0x1p100 ? 0u : 1u;
+        for (uint32_t r = threadIdx.x; r < rows; r += blockDim.x) by_record[r] = plan.disc_to_origin[r] < 0x1p100 ? 0u : ~0u;
     __syncthreads();
     if constexpr (kStaged) {
         for (uint32_t i = threadIdx.x; i < S * rows; i += blockDim.x) {
             const uint32_t k = i / rows, r = i % rows;
             ExerciseRule rule = never_exercise();
             if (int(k) < ns && r + 1 < rows) load_rule<kReadOnly>(&a.rules[sm.rbase[k] + r], &rule);
-            if (rule.general) by_record[r] = 1u;
+            if (rule.general) {
+                atomicOr(&by_record[r], 1u << k);
+                rule = never_exercise();
+            }
             StrikeRule& to = staged[r * S + k];
             to.slope = rule.slope;
             to.shift = rule.shift;
@@ -694,15 +698,22 @@ __device__ void evaluate_item(const BatchArgs& a, uint32_t gi, uint32_t first, u
                 }
                 return;
             }
-            if (!kStaged || by_record[row] != 0 || !within_rule(spot)) {
-                unsigned open = 0;
+            // The strikes of `apart` that still run, one by one: those without a staged rule, and every strike at a
+            // state or a discount beyond what the rules cover.
+            const auto decide_apart = [&](unsigned apart) {
 #pragma unroll
-                for (int k = 0; k < S; ++k) open |= running(k) ? 1u << k : 0u;
+                for (int k = 0; k < S; ++k) apart &= running(k) ? ~0u : ~(1u << k);
 #pragma unroll 1
                 for (int k = 0; k < ns; ++k) {
                     const double d = spot - sm.strikes[k];
-                    if (!((open >> k) & 1u) || !(d > 0.0)) continue;
-                    const int decision = decide_record<D>(a, sm.rbase[k] + row, spot, sm.strikes[k]);
+                    if (!((apart >> k) & 1u) || !(d > 0.0)) continue;
+                    int decision = kDecideContinue;
+                    const volatile ExerciseRule& rule = a.rules[sm.rbase[k] + row];  // read through L2
+                    if (!kStaged && rule.general == 0 && within_rule(spot) && disc < 0x1p100) {
+                        if (exercise_rule(a.tie_rule, d, rule_continuation<D>(rule, d))) decision = kDecideExercise;
+                    } else {
+                        decision = decide_record<D>(a, sm.rbase[k] + row, spot, sm.strikes[k]);
+                    }
                     ProblemStatus& st = a.problem_status[sm.problem[k]];
                     if (decision == kDecideNonFinite)
                         atomicMin(&st.eval_fail, ((unsigned long long)row << 33) | (p << 1));
@@ -712,11 +723,15 @@ __device__ void evaluate_item(const BatchArgs& a, uint32_t gi, uint32_t first, u
 #pragma unroll
                     for (int m = 0; m < S; ++m) payoff[m] = m == k ? fo_fabs(paid) : payoff[m];
                 }
-                return;
+            };
+            if (!kStaged || by_record[row] != 0 || !within_rule(spot)) {
+                const unsigned apart = kStaged && within_rule(spot) ? by_record[row] : ~0u;
+                decide_apart(apart);
+                if (S == 1 || apart == ~0u) return;
             }
-            // Every strike by the signs of K - spot, of the continuation less the excess and of the payoff so
-            // far: a strike without a rule never exercises. (A difference of finite doubles is zero, and
-            // then positive, only where they are equal.)
+            // The others by the signs of K - spot, of the continuation less the excess and of the payoff so far: a
+            // strike without a rule never exercises. (A difference of finite doubles is zero, and then
+            // positive, only where they are equal.)
             const StrikeRule* rules = staged + row * S;
             const auto decide = [&](auto strict) {
 #pragma unroll
@@ -1066,10 +1081,11 @@ __device__ __forceinline__ uint32_t dynamic_smem_bytes() {
 }
 
 // S: strikes an evaluation item applies together (kGreeks: one, with the adjoint). The dynamic
-// shared memory holds the staged rules (rule_rows x S ExerciseRules, plus one word per row: whether the row
-// needs its records, or its stopping count with the Greeks) when stage_rules is set; the fit kernel's
-// holds path values.
-template <int kPhase, int S, bool kGreeks, int D>
+// shared memory holds the staged rules (rule_rows x S ExerciseRules, plus one word per row: the strikes
+// that need their records, or its stopping count with the Greeks) when stage_rules is set; the fit kernel's
+// holds path values. kUnstaged: the evaluation kernel of the phase executor for launches that do not stage
+// (the staged form's steps keep the registers that this one's would take).
+template <int kPhase, int S, bool kGreeks, int D, bool kUnstaged>
 __global__ void __launch_bounds__(kPersistentThreads, (PhaseOccupancy<kPhase, S, kGreeks>::value))
     batch_persistent_kernel(BatchArgs a, BatchQueue q, uint32_t rule_rows, int stage_rules) {
     constexpr bool kSim = kPhase == kPhaseAll || kPhase == kPhaseSimulate;
@@ -1141,12 +1157,15 @@ __global__ void __launch_bounds__(kPersistentThreads, (PhaseOccupancy<kPhase, S,
                 } else {
                     constexpr bool kRO = kPhase == kPhaseEvaluate;
                     StrikeRule* rules = reinterpret_cast<StrikeRule*>(persistent_dyn);
-                    if (stage_rules)
-                        evaluate_item<S, D, true, kRO>(a, gi, it.first, it.count, it.chunk, normals, keys[1], sm.eval, rules,
-                                                       rule_rows);
-                    else
-                        evaluate_item<S, D, false, kRO>(a, gi, it.first, it.count, it.chunk, normals, keys[1], sm.eval, rules,
-                                                        rule_rows);
+                    constexpr bool kBoth = kPhase == kPhaseAll;
+                    if constexpr (kBoth || !kUnstaged)
+                        if (!kBoth || stage_rules)
+                            evaluate_item<S, D, true, kRO>(a, gi, it.first, it.count, it.chunk, normals, keys[1], sm.eval,
+                                                           rules, rule_rows);
+                    if constexpr (kBoth || kUnstaged)
+                        if (!kBoth || !stage_rules)
+                            evaluate_item<S, D, false, kRO>(a, gi, it.first, it.count, it.chunk, normals, keys[1], sm.eval,
+                                                            rules, rule_rows);
                 }
             }
             // The item that completes the group's evaluation writes the group's summaries (in the
@@ -1169,10 +1188,12 @@ __global__ void __launch_bounds__(kPersistentThreads, (PhaseOccupancy<kPhase, S,
 
 // ---- launcher ---------------------------------------------------------------------------------------
 
-template <int kPhase, int S, bool kGreeks, int D>
+template <int kPhase, int S, bool kGreeks, int D, bool kUnstaged = false>
 static cudaError_t prepare_persistent_d(const BatchQueue& q, uint32_t rule_rows, bool stage, int ctas_per_sm,
                                         PersistentLaunch* out) {
-    auto kernel = batch_persistent_kernel<kPhase, S, kGreeks, D>;
+    if constexpr (kPhase == kPhaseEvaluate && !kGreeks && !kUnstaged)
+        if (!stage) return prepare_persistent_d<kPhase, S, kGreeks, D, true>(q, rule_rows, stage, ctas_per_sm, out);
+    auto kernel = batch_persistent_kernel<kPhase, S, kGreeks, D, kUnstaged>;
     const bool rules = stage && (kPhase == kPhaseAll || kPhase == kPhaseEvaluate);
     size_t smem = rules ? persistent_rule_bytes(S, kGreeks, rule_rows) : 0;
     if (kPhase == kPhaseFit) {
