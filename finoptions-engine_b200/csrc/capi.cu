@@ -36,7 +36,7 @@ struct PlanLayout {
     size_t sqrt_dt, dt;       // per-interval sqrt(dt) and dt for the adjoint vega
     size_t greek_partials;    // eval_blocks * kGreekSlots double2
     size_t greek_out;         // kGreekSlots doubles (read back)
-    size_t partials;          // exchange buffers of the backward pass (at most 2 * blocks * 16 double2)
+    size_t partials;          // exchange buffers of the backward pass (exchange_words double2)
     size_t eval_partials;     // eval partials: eval_blocks * 2 double2
     size_t out;               // start of the read-back region
     size_t status, result, records, counts, itm_counts, replay;
@@ -153,7 +153,7 @@ PlanLayout layout_for(const HostPlan& hp, int backward_blocks, int eval_blocks) 
     L.sqrt_dt = take(sizeof(double) * std::max<size_t>(hp.intervals(), 1));
     L.dt = take(sizeof(double) * std::max<size_t>(hp.intervals(), 1));
     L.inputs_bytes = off;
-    L.partials = take(sizeof(double2) * 2 * size_t(backward_blocks) * 16);
+    L.partials = take(sizeof(double2) * size_t(exchange_words(backward_blocks)));
     L.eval_partials = take(sizeof(double2) * size_t(eval_blocks) * 2);
     L.greek_partials = take(sizeof(double2) * size_t(eval_blocks) * kGreekSlots);
     off = align_up(off, 256);
