@@ -34,7 +34,8 @@ constexpr unsigned long long kNone = ~0ull;
 struct PlanLayout {
     size_t steps, events, row_node, disc_from_later, disc_to_origin, escrow_cash;  // inputs
     size_t sqrt_dt, dt;       // per-interval sqrt(dt) and dt for the adjoint vega
-    size_t greek_partials;    // eval_blocks * kGreekSlots double2
+    size_t greek_partials;    // eval_blocks * kGreekSlots double2; before the evaluation the moments' workspace
+    size_t workspace_bytes;   // its size
     size_t greek_out;         // kGreekSlots doubles (read back)
     size_t partials;          // exchange buffers of the backward pass (exchange_words double2)
     size_t eval_partials;     // eval partials: eval_blocks * 2 double2
@@ -134,7 +135,7 @@ Error choose_backward_shape(const fo_executor* ex, uint64_t paths, int* blocks, 
     return Error{};
 }
 
-PlanLayout layout_for(const HostPlan& hp, int backward_blocks, int eval_blocks) {
+PlanLayout layout_for(const HostPlan& hp, int backward_blocks, int eval_blocks, size_t moment_bytes) {
     PlanLayout L{};
     size_t off = 0;
     auto take = [&](size_t bytes) {
@@ -155,7 +156,8 @@ PlanLayout layout_for(const HostPlan& hp, int backward_blocks, int eval_blocks) 
     L.inputs_bytes = off;
     L.partials = take(sizeof(double2) * size_t(exchange_words(backward_blocks)));
     L.eval_partials = take(sizeof(double2) * size_t(eval_blocks) * 2);
-    L.greek_partials = take(sizeof(double2) * size_t(eval_blocks) * kGreekSlots);
+    L.workspace_bytes = std::max(sizeof(double2) * size_t(eval_blocks) * kGreekSlots, moment_bytes);
+    L.greek_partials = take(L.workspace_bytes);
     off = align_up(off, 256);
     L.out = off;
     L.status = take(sizeof(DeviceStatus));
@@ -168,6 +170,18 @@ PlanLayout layout_for(const HostPlan& hp, int backward_blocks, int eval_blocks) 
     L.out_bytes = align_up(off, 256) - L.out;
     L.total = align_up(off, 256);
     return L;
+}
+
+// Rows whose moments are reduced ahead of the backward pass.
+uint32_t fitted_rows(const HostPlan& hp) { return hp.rows() - 1 - (hp.origin_row ? 1u : 0u); }
+
+// Workspace in which every CTA of the moments launch finds room for its totals (none with one CTA a row).
+// A small evaluation beside a large training population has fewer partials of its own: 12 dates, 3,000,001
+// training and 4,096 evaluation paths took 1,985 us a call with the CTAs that fit among those.
+size_t moment_workspace(const HostPlan& hp, int sms) {
+    const uint32_t rows = fitted_rows(hp);
+    const int blocks = rows > 0 ? moment_blocks(hp.train_paths, rows, sms, SIZE_MAX) : 1;
+    return blocks > 1 ? moment_workspace_bytes(rows, blocks) : 0;
 }
 
 // Packs the plan arrays in the same layout as the device block's input region.
@@ -263,7 +277,7 @@ Error plan_create(fo_executor* ex, const fo_lsm_call_request& q, bool own_memory
     const uint64_t eval_needed = plan->run_eval ? (hp.eval_paths + eval_threads - 1) / eval_threads : 1;
     plan->eval_blocks = int(std::max<uint64_t>(1, std::min<uint64_t>(eval_needed, uint64_t(ex->sms) * ex->eval_blocks_per_sm)));
     plan->first_stored_row = hp.origin_row ? 1u : 0u;
-    plan->lay = layout_for(hp, plan->backward_blocks, plan->eval_blocks);
+    plan->lay = layout_for(hp, plan->backward_blocks, plan->eval_blocks, moment_workspace(hp, ex->sms));
     const PlanLayout& L = plan->lay;
     // device memory: plan block + slab
     if (own_memory) {
@@ -338,10 +352,9 @@ Error plan_launch(fo_lsm_call_plan* plan) {
     mo.status = status;
     mo.exchange = reinterpret_cast<double2*>(dev + L.partials);
     mo.exchange_words = exchange_words(plan->backward_blocks);
-    const uint32_t fitted_rows = plan->hp.rows() - 1 - (plan->hp.origin_row ? 1u : 0u);
-    if (fitted_rows > 0) {
-        const size_t workspace = sizeof(double2) * kGreekSlots * size_t(plan->eval_blocks);
-        FO_CUDA_TRY(launch_moments(mo, moment_blocks(plan->hp.train_paths, fitted_rows, ex->sms, workspace), s), "moments launch");
+    if (const uint32_t rows = fitted_rows(plan->hp); rows > 0) {
+        const int blocks = moment_blocks(plan->hp.train_paths, rows, ex->sms, L.workspace_bytes);
+        FO_CUDA_TRY(launch_moments(mo, blocks, s), "moments launch");
     } else {
         FO_CUDA_TRY(cudaMemsetAsync(mo.exchange, 0, sizeof(double2) * mo.exchange_words, s), "reset");
     }
@@ -866,7 +879,7 @@ Error simulate_gbm(fo_executor* executor, const fo_gbm_seeded_request& q, const 
     hp.initial_spot = s0;
     hp.disc_from_later.assign(rows, 1.0);
     hp.disc_to_origin.assign(rows, 1.0);
-    PlanLayout L = layout_for(hp, 1, 1);
+    PlanLayout L = layout_for(hp, 1, 1, 0);
     e = executor->scratch.reserve(L.total);
     if (e.ok()) e = executor->staging.reserve(std::max(L.inputs_bytes, L.out_bytes));
     if (e.ok() && !states_on_device) e = executor->slab.reserve(sizeof(double) * rows * paths);
@@ -1348,7 +1361,7 @@ Error price_noalloc(const fo_lsm_call_request& q, cudaStream_t stream, fo_lsm_ca
     const uint64_t eval_needed = plan.run_eval ? (hp.eval_paths + kEvalThreads - 1) / kEvalThreads : 1;
     plan.eval_blocks = int(std::max<uint64_t>(1, std::min<uint64_t>(eval_needed, uint64_t(shadow.sms) * 8)));
     plan.first_stored_row = hp.origin_row ? 1u : 0u;
-    plan.lay = layout_for(hp, plan.backward_blocks, plan.eval_blocks);
+    plan.lay = layout_for(hp, plan.backward_blocks, plan.eval_blocks, 0);
     const PlanLayout& L = plan.lay;
     const uint64_t stored_rows = hp.rows() - plan.first_stored_row;
     const uint64_t slab_bytes = uint64_t(sizeof(double)) * stored_rows * hp.train_paths +
@@ -1360,6 +1373,10 @@ Error price_noalloc(const fo_lsm_call_request& q, cudaStream_t stream, fo_lsm_ca
                               " bytes of device scratch; the allocation-free entry point holds at most " +
                               std::to_string(uint64_t(FO_NOALLOC_SCRATCH_BYTES)) +
                               " bytes (training paths x stored rows x 8 bytes plus the plan block)");
+    // The moments' workspace takes what the request leaves (their launch makes do with less).
+    plan.lay = layout_for(hp, plan.backward_blocks, plan.eval_blocks,
+                          std::min<size_t>(moment_workspace(hp, shadow.sms),
+                                           L.workspace_bytes + (FO_NOALLOC_SCRATCH_BYTES - needed) / 256 * 256));
     std::vector<unsigned char> host(std::max(L.inputs_bytes, L.out_bytes));
     plan.d_block = scratch;
     plan.d_slab = reinterpret_cast<double*>(scratch + L.total);

@@ -682,9 +682,11 @@ __global__ void __launch_bounds__(kBackwardThreads, 1) backward_kernel(BackwardA
 int moment_blocks(uint64_t paths, uint32_t rows, int sms, size_t workspace_bytes) {
     const uint64_t by_work = (paths + 2047) / 2048;
     const uint64_t by_device = uint64_t(sms) * kMomentCtasPerSm / rows;
-    const uint64_t by_space = workspace_bytes / (sizeof(double2) * kSlots * rows);
+    const uint64_t by_space = workspace_bytes / moment_workspace_bytes(rows, 1);
     return int(std::max<uint64_t>(1, std::min(std::min(by_work, by_device), by_space)));
 }
+
+size_t moment_workspace_bytes(uint32_t rows, int blocks) { return sizeof(double2) * kSlots * rows * size_t(blocks); }
 
 template <int D>
 static cudaError_t launch_moments_d(const MomentArgs& args, int rows, int blocks, cudaStream_t stream) {

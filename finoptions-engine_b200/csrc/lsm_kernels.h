@@ -108,7 +108,9 @@ cudaError_t launch_simulate_external(const DevicePlan& plan, uint64_t paths, con
                                      unsigned long long* fail, cudaStream_t stream);
 cudaError_t launch_replay_external(const DevicePlan& plan, uint64_t paths, const double* normals, uint64_t path,
                                    SimFailure* out, cudaStream_t stream);
+// CTAs per row of the moments launch, at most what the workspace holds; what that many take.
 int moment_blocks(uint64_t paths, uint32_t rows, int sms, size_t workspace_bytes);
+size_t moment_workspace_bytes(uint32_t rows, int blocks);
 cudaError_t launch_moments(const MomentArgs& args, int blocks, cudaStream_t stream);
 int backward_max_blocks(int device);
 int backward_max_ppt();
