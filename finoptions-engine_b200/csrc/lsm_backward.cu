@@ -75,13 +75,16 @@ __device__ __forceinline__ double moneyness(double spot, const Divisor& strike) 
 // A grid of a.blocks CTAs per row, each over a contiguous range of paths; a row's last CTA adds the
 // CTA totals in order, solves the row (lsm_fit_warp.cuh with zero responses) and writes its record.
 // The power sums are taken about the in-the-money mean of the row's first thousand paths, which
-// lies within a fraction of a standard deviation of the row's; where it does not (a few
-// in-the-money paths), the last CTA takes the row's sums again about its own mean.
+// lies within a fraction of a standard deviation of the row's. Where it does not (a few in-the-money
+// paths), the row's sums are taken again about its own mean: by the last CTA alone, or, for more than
+// kRetakePaths paths, by a second launch (kAgain), whose CTAs leave at once for every other row. 52
+// weeks, 2^20 paths, strike at 1.6 times the spot: 1,906 us a call by the last CTA, 1,308 so.
 // It reads the stored rows once, at about half the FP64 rate and half of HBM's: 2^20 paths x 51 rows take
 // 137 us, 200 us with the quotient formed for each path and every power added by itself.
 constexpr int kMomentThreads = 256;
 constexpr int kMomentCtasPerSm = 4;
 constexpr int kPivotLoads = 4;  // the pivot's sample: the row's first kPivotLoads * kMomentThreads paths
+constexpr uint64_t kRetakePaths = 1 << 17;  // one CTA reads this many in 80 us, the second launch takes 4
 constexpr int kHugeSlot = kBadSlot + 1;  // in-the-money paths beyond kRuleSpotLimit
 
 // A path's t = spot / strike - pivot is one fma with the strike's reciprocal: the same affine map of every
@@ -130,14 +133,14 @@ __device__ __forceinline__ void add_row_moments(RowSums& s, uint32_t& itm, const
     }
 }
 
-template <int D>
+template <int D, bool kAgain>
 __global__ void __launch_bounds__(kMomentThreads, kMomentCtasPerSm) moments_kernel(MomentArgs a) {
     __shared__ double red[32 * kSlots];
     __shared__ dd total[kSlots];
     __shared__ FitModel model;
     __shared__ int last;
     const DevicePlan& plan = a.plan;
-    if (blockIdx.x == 0 && blockIdx.y == 0)
+    if (!kAgain && blockIdx.x == 0 && blockIdx.y == 0)
         for (int i = threadIdx.x; i < a.exchange_words; i += blockDim.x) a.exchange[i] = make_double2(0.0, 0.0);
     if (*(const volatile unsigned long long*)&a.status->train_sim_fail != kNone) return;
     const uint32_t E = plan.rows - 1;
@@ -148,7 +151,10 @@ __global__ void __launch_bounds__(kMomentThreads, kMomentCtasPerSm) moments_kern
     const Divisor Kd = make_divisor(plan.strike);
     FitRecord& rec = a.records[row];
     double pivot = 1.0;
-    if constexpr (D > 0) {
+    if constexpr (kAgain) {
+        if (rec.again == 0) return;
+        pivot = rec.pivot;
+    } else if constexpr (D > 0) {
         double loc[2] = {0.0, 0.0}, sample[kPivotLoads];
 #pragma unroll
         for (int u = 0; u < kPivotLoads; ++u) {
@@ -173,7 +179,7 @@ __global__ void __launch_bounds__(kMomentThreads, kMomentCtasPerSm) moments_kern
     uint32_t itm_paths = 0;
     const uint64_t span = (P + gridDim.x - 1) / gridDim.x;
     const uint64_t lo = min(P, span * blockIdx.x), hi = min(P, lo + span);
-    add_row_moments<D>(s, itm_paths, spots, lo, hi, Kd, pivot, order, &a.status->fit_nonfinite);
+    add_row_moments<D>(s, itm_paths, spots, lo, hi, Kd, pivot, order, kAgain ? nullptr : &a.status->fit_nonfinite);
     s.acc[0] = double(itm_paths);
     cta_reduce_dd<kSlots>(s.acc, red, total);
     if (gridDim.x > 1) {
@@ -202,8 +208,16 @@ __global__ void __launch_bounds__(kMomentThreads, kMomentCtasPerSm) moments_kern
     const bool huge = total[kHugeSlot].hi > 0.0;
     const uint32_t required = uint32_t(D + 1);
     double mean = pivot;
-    if (D > 0 && population >= required && bad == 0 && pivot_too_far(total, pivot, itm, &mean)) {
+    if (!kAgain && D > 0 && population >= required && bad == 0 && pivot_too_far(total, pivot, itm, &mean)) {
         pivot = mean;
+        if (P > kRetakePaths) {
+            if (threadIdx.x == 0) {
+                rec.pivot = pivot;
+                rec.arrived = 0;
+                rec.again = 1;
+            }
+            return;
+        }
 #pragma unroll
         for (int k = 0; k < kSlots; ++k) s.acc[k] = 0.0;
         itm_paths = 0;
@@ -692,7 +706,10 @@ template <int D>
 static cudaError_t launch_moments_d(const MomentArgs& args, int rows, int blocks, cudaStream_t stream) {
     // Not by launch_early: with an event recorded behind it for another stream, a call took 25 us more (52 weeks,
     // 2^20 paths: 1,250 us against 1,218).
-    moments_kernel<D><<<dim3(unsigned(blocks), unsigned(rows)), kMomentThreads, 0, stream>>>(args);
+    const dim3 grid{unsigned(blocks), unsigned(rows)};
+    moments_kernel<D, false><<<grid, kMomentThreads, 0, stream>>>(args);
+    if constexpr (D > 0)
+        if (args.plan.train_paths > kRetakePaths) moments_kernel<D, true><<<grid, kMomentThreads, 0, stream>>>(args);
     return cudaGetLastError();
 }
 

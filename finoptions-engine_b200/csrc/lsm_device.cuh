@@ -52,6 +52,7 @@ struct FitRecord {
     int32_t diag_aux;
     int32_t beyond_rule;     // a training spot lies beyond kRuleSpotLimit (single contracts)
     uint32_t arrived;        // CTAs whose moments of the row are in (single contracts)
+    int32_t again;           // the row's moments are to be taken again about `pivot` (single contracts)
 };
 
 // Device status words. Path-addressed failures keep the lowest key with atomicMin so the host

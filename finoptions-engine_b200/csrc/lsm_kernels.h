@@ -20,7 +20,7 @@ struct MomentArgs {
     DevicePlan plan;
     const double* slab;          // stored training rows [rows - first_stored_row, paths]
     double2* partials;           // [fitted rows][blocks][16] CTA totals (unused with one block a row)
-    FitRecord* records;          // [rows]; `arrived` starts at zero
+    FitRecord* records;          // [rows]; `arrived` and `again` start at zero
     DeviceStatus* status;
     double2* exchange;           // BackwardArgs::partials
     int exchange_words;          // exchange_words(backward blocks)
