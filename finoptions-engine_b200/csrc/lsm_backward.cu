@@ -12,42 +12,16 @@
 #include <algorithm>
 #include <type_traits>
 
+#include "lsm_bulk_copy.cuh"
 #include "lsm_common.cuh"
 #include "lsm_device.cuh"
+#include "lsm_exchange.cuh"
 #include "lsm_fit_warp.cuh"
 #include "lsm_kernels.h"
 #include "lsm_row_solve.cuh"
 #include "lsm_sync.cuh"
 
 namespace fo {
-
-// One bulk copy (TMA) per row and CTA, completed on an mbarrier. Source, destination and size are
-// multiples of 16 bytes (the caller rounds).
-__device__ __forceinline__ uint32_t shared_address(const void* p) { return uint32_t(__cvta_generic_to_shared(p)); }
-__device__ __forceinline__ void mbarrier_init(uint64_t* bar, uint32_t arrivals) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(shared_address(bar)), "r"(arrivals) : "memory");
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-__device__ __forceinline__ void bulk_load(void* smem, const void* gmem, uint32_t bytes, uint64_t* bar) {
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(shared_address(bar)), "r"(bytes)
-                 : "memory");
-    if (bytes > 0)
-        asm volatile(
-            "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                shared_address(smem)),
-            "l"(gmem), "r"(bytes), "r"(shared_address(bar))
-            : "memory");
-}
-__device__ __forceinline__ bool mbarrier_try_wait(uint64_t* bar, uint32_t parity) {
-    uint32_t done;
-    asm volatile(
-        "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
-        : "=r"(done)
-        : "r"(shared_address(bar)), "r"(parity)
-        : "memory");
-    return done != 0;
-}
 
 // Double-double sum over a warp in a fixed order, in lane 0. The low parts are summed beside the
 // high ones and folded in once, so a level costs a shuffle and one dependent addition.
@@ -256,128 +230,17 @@ __global__ void __launch_bounds__(kMomentThreads, kMomentCtasPerSm) moments_kern
 // The serial pass.
 // ---------------------------------------------------------------------------------------------
 
-constexpr int kExchangeSlots = 8;               // R_0..R_4, non-finite responses, spare
-constexpr int kBadResponses = kMaxColumns;
-constexpr int kUsedSlots = kMaxColumns + 1;
-constexpr int kExchangeWarps = 8;
-constexpr int kExchangeLoads = 5;                // CTA lines a lane reads together (148 CTAs: one round)
 constexpr int kFetchThread = (kExchangeWarps + 1) * 32;
+static_assert(kUsedSlots == kMaxColumns + 1, "R_0..R_4 and the non-finite responses");
+constexpr int kBadResponses = kMaxColumns;
 
 struct BackwardSmem {
-    double red[kBackwardThreads / 32][kExchangeSlots];  // per warp and slot
-    dd share[kExchangeWarps][kExchangeSlots];  // the exchange warps' shares of the grid's totals
+    ExchangeSmem<kBackwardThreads / 32> exchange;
     RowBasis basis[2];  // of the row being decided and of the row being staged, by row parity
     RowSolution row;    // of the row being decided
-    int failed;       // a wait timed out
+    int failed;         // the wait for a copy timed out
     uint64_t loaded;  // mbarrier of the staged row's spots
 };
-
-// Grid-wide sums. A CTA's totals travel as one line of eight 16-byte double-doubles whose lowest bits are
-// the exchange's phase (moving hi's lowest bit into lo costs nothing, lo loses 2^-105 of the sum), so
-// a reader that sees the phase in both halves has the value: no counter is written, fenced and
-// waited for first. Two buffers alternate and a buffer's phase flips each time it is reused; a CTA
-// writes exchange s + 2 only after reading s + 1 from every CTA, which each wrote only after it
-// had read s.
-__device__ __forceinline__ double2 with_phase(dd v, uint64_t phase) {
-    const double hi = bits_to_double((double_to_bits(v.hi) & ~1ull) | phase);
-    const double lo = v.lo + (v.hi - hi);
-    return make_double2(hi, bits_to_double((double_to_bits(lo) & ~1ull) | phase));
-}
-__device__ __forceinline__ void store_relaxed(double2* p, double2 v) {
-    asm volatile("st.relaxed.gpu.global.v2.f64 [%0], {%1, %2};" ::"l"(p), "d"(v.x), "d"(v.y) : "memory");
-}
-__device__ __forceinline__ double2 load_relaxed(const double2* p) {
-    double2 v;
-    asm volatile("ld.relaxed.gpu.global.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p) : "memory");
-    return v;
-}
-__device__ __forceinline__ bool has_phase(double2 v, uint64_t phase) {
-    return (double_to_bits(v.x) & 1ull) == phase && (double_to_bits(v.y) & 1ull) == phase;
-}
-// Adds a double-double to a running sum whose parts are renormalised once at the end: the chain of
-// high parts is one addition a step.
-__device__ __forceinline__ void add_to(dd& sum, dd v) {
-    const dd s = two_sum(sum.hi, v.hi);
-    sum.hi = s.hi;
-    sum.lo = (sum.lo + v.lo) + s.lo;
-}
-__device__ __forceinline__ dd shfl_dd_xor(dd v, int mask) {
-    return dd{__shfl_xor_sync(0xffffffffu, v.hi, mask), __shfl_xor_sync(0xffffffffu, v.lo, mask)};
-}
-// Sums over the four lanes that hold the same slot (lane & 7); every lane ends with its slot's sum.
-__device__ __forceinline__ dd slot_sum(dd v) {
-    // The lower lane's value first on both sides, so that both form the same sum.
-#pragma unroll
-    for (int mask = kExchangeSlots; mask < 32; mask <<= 1) {
-        const dd o = shfl_dd_xor(v, mask);
-        const bool upper = (threadIdx.x & mask) != 0;
-        dd first = upper ? o : v;
-        add_to(first, upper ? v : o);
-        v = first;
-    }
-    return fast_two_sum(v.hi, v.lo);
-}
-
-// The grid's totals from the CTA's per-warp sums (sm.red), by the first kExchangeWarps warps, which meet
-// at named barrier 1: warp 0 sends this CTA's totals, all read the others', and warp 0 adds the
-// warps' shares. Returns slot (lane & 7) in every lane of warp 0. sm.failed is set when a wait gave up.
-__device__ __forceinline__ dd exchange_totals(const BackwardArgs& a, BackwardSmem& sm, unsigned seq) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int slot = lane & (kExchangeSlots - 1), blocks = int(gridDim.x);
-    double2* buffer = a.partials + size_t(seq & 1u) * kExchangeSlots * blocks;
-    const uint64_t phase = ((seq >> 1) & 1u) ^ 1u;  // the buffers start at phase 0
-    dd total = dd_make(0.0);
-    if (warp == 0) {
-        constexpr int kShare = kBackwardThreads / 32 * kExchangeSlots / 32;  // warp sums a lane adds
-        double mine[kShare];
-#pragma unroll
-        for (int i = 0; i < kShare; ++i) mine[i] = sm.red[lane / kExchangeSlots + i * (32 / kExchangeSlots)][slot];
-#pragma unroll
-        for (int i = 0; i < kShare; ++i) add_to(total, dd_make(mine[i]));
-        total = slot_sum(total);
-        if (blocks > 1 && lane < kUsedSlots)
-            store_relaxed(&buffer[size_t(blockIdx.x) * kExchangeSlots + slot], with_phase(total, phase));
-    }
-    if (blocks == 1) return total;
-    dd sum = dd_make(0.0);
-    constexpr int kCtasPerWarp = 32 / kExchangeSlots, kRound = kExchangeWarps * kCtasPerWarp;
-    for (int first = 0; first < blocks; first += kRound * kExchangeLoads) {
-        double2 v[kExchangeLoads];
-        unsigned missing = 0;  // loads of this lane without their value yet
-#pragma unroll
-        for (int i = 0; i < kExchangeLoads; ++i) {
-            const int b = first + i * kRound + warp * kCtasPerWarp + lane / kExchangeSlots;
-            v[i] = make_double2(0.0, 0.0);
-            if (b < blocks && slot < kUsedSlots) missing |= 1u << i;
-        }
-        BoundedWait wait(a.status);
-        for (;;) {
-#pragma unroll
-            for (int i = 0; i < kExchangeLoads; ++i) {
-                const int b = first + i * kRound + warp * kCtasPerWarp + lane / kExchangeSlots;
-                if ((missing >> i) & 1u) v[i] = load_relaxed(&buffer[size_t(b) * kExchangeSlots + slot]);
-            }
-#pragma unroll
-            for (int i = 0; i < kExchangeLoads; ++i)
-                if (has_phase(v[i], phase)) missing &= ~(1u << i);
-            if (__all_sync(0xffffffffu, missing == 0)) break;
-            if (!wait.again()) {
-                if (lane == 0) sm.failed = 1;
-                break;
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < kExchangeLoads; ++i) add_to(sum, dd{v[i].x, v[i].y});
-    }
-    sum = slot_sum(sum);
-    if (lane < kExchangeSlots) sm.share[warp][slot] = sum;
-    named_barrier_sync(1, kExchangeWarps * 32);
-    if (warp != 0) return sum;
-    dd grid = sm.share[lane / kExchangeSlots][slot];
-    add_to(grid, sm.share[lane / kExchangeSlots + 4][slot]);
-    static_assert(kExchangeWarps == 8 && kExchangeSlots == 8, "two shares a lane");
-    return slot_sum(grid);
-}
 
 // The row's coefficients into its record, by one warp of CTA 0; and the failure of a row whose response sums
 // leave no finite coefficient.
@@ -445,6 +308,7 @@ __global__ void __launch_bounds__(kBackwardThreads, 1) backward_kernel(BackwardA
     }
     if (threadIdx.x == 0) {
         sm.failed = 0;
+        sm.exchange.failed = 0;
         sm.row.rule = never_exercise();
         mbarrier_init(&sm.loaded, 1);
     }
@@ -469,12 +333,7 @@ __global__ void __launch_bounds__(kBackwardThreads, 1) backward_kernel(BackwardA
     uint32_t copies = 0;  // completed copies
     auto wait_copy = [&] {
         if constexpr (!kHbm) {
-            for (int tries = 0; !mbarrier_try_wait(&sm.loaded, copies & 1u); ++tries) {
-                if (tries < (1 << 22)) continue;
-                atomicExch(&a.status->barrier_timeout, 1u);
-                sm.failed = 1;
-                break;
-            }
+            if (!wait_bulk(&sm.loaded, copies & 1u, a.status)) sm.failed = 1;
             copies += 1;
         }
     };
@@ -597,10 +456,10 @@ __global__ void __launch_bounds__(kBackwardThreads, 1) backward_kernel(BackwardA
             value(j) = v;
         }
     };
-    // The thread's sums to sm.red, slot by slot.
+    // The thread's sums to sm.exchange.red, slot by slot.
     auto reduce_warps = [&] {
         const double total = warp_transpose_reduce<kExchangeSlots>(sums);
-        if (lane < kExchangeSlots) sm.red[warp][lane] = total;
+        if (lane < kExchangeSlots) sm.exchange.red[warp][lane] = total;
         clear_sums();
     };
     const auto prepare = [&](int at) {
@@ -636,7 +495,7 @@ __global__ void __launch_bounds__(kBackwardThreads, 1) backward_kernel(BackwardA
         __syncthreads();
         if (warp < kExchangeWarps) {
             if (fits) {
-                const double total = dd_round(exchange_totals(a, sm, seq));
+                const double total = dd_round(exchange_totals(sm.exchange, a.partials, int(blockIdx.x), int(gridDim.x), seq, a.status));
                 if (warp == 0)
                     solve_row<D>(basis, total, __shfl_sync(0xffffffffu, total, kBadResponses) > 0.5, &sm.row);
             } else if (threadIdx.x == 0) {
@@ -651,7 +510,7 @@ __global__ void __launch_bounds__(kBackwardThreads, 1) backward_kernel(BackwardA
             }
         }
         __syncthreads();
-        if (sm.failed) return;
+        if (sm.failed != 0 || sm.exchange.failed != 0) return;
         if (fits && blockIdx.x == 0 && warp == kExchangeWarps) write_coefficients<D>(sm.row, a.records[row]);
         if (sm.row.kind == kRuleFitFailed) {
             if (blockIdx.x == 0 && threadIdx.x == 0) atomicMin(&a.status->fit_failed_order, order);
@@ -672,8 +531,8 @@ __global__ void __launch_bounds__(kBackwardThreads, 1) backward_kernel(BackwardA
         reduce_warps();
         __syncthreads();
         dd total = dd_make(0.0);
-        if (warp < kExchangeWarps) total = exchange_totals(a, sm, seq);
-        if (blockIdx.x == 0 && threadIdx.x == 0 && sm.failed == 0) {
+        if (warp < kExchangeWarps) total = exchange_totals(sm.exchange, a.partials, int(blockIdx.x), int(gridDim.x), seq, a.status);
+        if (blockIdx.x == 0 && threadIdx.x == 0 && sm.exchange.failed == 0) {
             const double mean = dd_round(dd_div(total, dd_make(double(P))));
             const double intrinsic = plan.initial_spot - K > 0.0 ? plan.initial_spot - K : 0.0;
             FitRecord& rec = a.records[0];

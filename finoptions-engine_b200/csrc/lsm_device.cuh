@@ -68,7 +68,7 @@ struct DeviceStatus {
     unsigned long long fit_nonfinite;    // (order << 32) | path: non-finite ITM predictor/response
     unsigned int fit_failed_order;       // first backward order whose fit failed
     unsigned int barrier_timeout;        // zero-initialised: a grid wait timed out
-    unsigned int arrivals;               // zero-initialised: what wait_arrivals counts
+    unsigned int arrivals;               // zero between launches: CTAs of the evaluation that are done (last_cta)
 };
 constexpr size_t kStatusNoneBytes = 7 * sizeof(unsigned long long) + sizeof(unsigned int);
 

@@ -61,8 +61,9 @@ struct BoundedWait {
     }
 };
 
-// Warp-wide wait until the arrival counter reaches `target`: lane 0 reads it and every decision is taken
-// on its broadcast value. False (in every lane) when the wait gave up.
+// Warp-wide wait until status->arrivals reaches `target`: lane 0 reads it and every decision is taken on its
+// broadcast value. False (in every lane) when the wait gave up. No kernel of the engine counts arrivals
+// between CTAs any more (lsm_exchange.cuh polls the values themselves); the bounded-wait test runs it.
 __device__ inline bool wait_arrivals(DeviceStatus* st, unsigned target,
                                      unsigned long long limit_ns = kBarrierTimeoutNs) {
     BoundedWait wait(st, limit_ns);
