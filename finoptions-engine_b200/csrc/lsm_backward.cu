@@ -54,21 +54,22 @@ __device__ __forceinline__ double moneyness(double spot, const Divisor& strike) 
 // kRetakePaths paths, by a second launch (kAgain), whose CTAs leave at once for every other row. 52
 // weeks, 2^20 paths, strike at 1.6 times the spot: 1,906 us a call by the last CTA, 1,308 so.
 // It reads the stored rows once, at about half the FP64 rate and half of HBM's: 2^20 paths x 51 rows take
-// 137 us, 200 us with the quotient formed for each path and every power added by itself.
+// 143 us, 200 us with every power added by itself.
 constexpr int kMomentThreads = 256;
 constexpr int kMomentCtasPerSm = 4;
 constexpr int kPivotLoads = 4;  // the pivot's sample: the row's first kPivotLoads * kMomentThreads paths
 constexpr uint64_t kRetakePaths = 1 << 17;  // one CTA reads this many in 80 us, the second launch takes 4
 constexpr int kHugeSlot = kBadSlot + 1;  // in-the-money paths beyond kRuleSpotLimit
 
-// A path's t = spot / strike - pivot is one fma with the strike's reciprocal: the same affine map of every
-// spot, so the regression on it is the regression on the quotients, with one rounding less a path.
+// A path's t is its correctly rounded quotient by the strike less the pivot. (One fma with the strike's
+// reciprocal takes 10 us less at 2^20 paths x 51 rows, but shifts every path, and so the recorded mean,
+// by the reciprocal's rounding.)
 template <int D>
 __device__ __forceinline__ void add_row_moments(RowSums& s, uint32_t& itm, const double* spots, uint64_t lo, uint64_t hi,
                                                 const Divisor& Kd, double pivot, uint32_t order,
                                                 unsigned long long* nonfinite) {
     constexpr int kLoads = 4;
-    const bool exact = Kd.inv == 0.0;  // no reciprocal: divide
+    const bool divides = !(Kd.b > 0x1p-800);  // a quotient could overflow, or there is no reciprocal
     for (uint64_t base = lo + threadIdx.x; base < hi; base += kLoads * kMomentThreads) {
         double sp[kLoads];
 #pragma unroll
@@ -79,18 +80,18 @@ __device__ __forceinline__ void add_row_moments(RowSums& s, uint32_t& itm, const
 #pragma unroll
         for (int u = 0; u < kLoads; ++u) {
             if (!(sp[u] > Kd.b)) continue;
-            double t = fo_fma(sp[u], Kd.inv, -pivot);
-            if (exact || !within_rule(sp[u])) {
-                const double x = sp[u] / Kd.b;
+            double x = divide_above(sp[u], Kd);
+            if (divides || !within_rule(sp[u])) {
+                x = sp[u] / Kd.b;
                 if (!finite_nonnegative(x)) {
                     s.acc[kBadSlot] += 1.0;
                     if (nonfinite)
                         atomicMin(nonfinite, ((unsigned long long)order << 32) | (base + uint64_t(u) * kMomentThreads));
                     continue;
                 }
-                t = x - pivot;
                 if (!within_rule(sp[u])) s.acc[kHugeSlot] += 1.0;
             }
+            const double t = x - pivot;
             itm += 1;
             // T_1 .. T_2D: the powers up to t^D are formed, the higher ones are products of two of them
             // added in one fma.
