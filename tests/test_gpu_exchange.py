@@ -7,6 +7,7 @@ one CTA whose neighbours' lines the host lays out.
 from __future__ import annotations
 
 import ctypes
+import math
 import subprocess
 from pathlib import Path
 
@@ -73,6 +74,21 @@ def test_the_grid_total_is_the_sum_of_the_lines(harness, blocks, seq) -> None:
     out, flag = exchange(harness, sums[1], grid_lines(harness, sums, 1, seq), 1, seq)
     assert out["failed"] == 0 and flag == 0 and out["warps_left"] == WARPS
     np.testing.assert_array_equal(out["total"].sum(axis=1)[:USED], sums.sum(axis=(0, 1))[:USED])
+
+
+@pytest.mark.parametrize("blocks, spread, signs", [(148, 2, False), (148, 30, False), (98, 2, True), (37, 20, True)])
+def test_the_grid_total_rounds_to_the_exact_sum(harness, blocks, spread, signs) -> None:
+    # Warp sums spread over 2 to 30 binary orders, of one sign or cancelling to a thousandth of their sum and
+    # less: the exchanged total, of some 100 bits, rounds to the binary64 number nearest to the exact sum.
+    rng = np.random.default_rng(spread + blocks)
+    for seq in range(4):
+        sums = np.exp2(rng.uniform(0.0, spread, (blocks, WARPS, SLOTS))) * rng.uniform(1.0, 2.0, (blocks, WARPS, SLOTS))
+        if signs:
+            sums[1::2] = -sums[0::2][: blocks // 2] * rng.uniform(0.999, 1.001, sums[1::2].shape)
+        out, flag = exchange(harness, sums[0], grid_lines(harness, sums, 0, seq), 0, seq)
+        assert out["failed"] == 0 and flag == 0
+        got = out["total"].sum(axis=1)[:USED]
+        assert got.tolist() == [math.fsum(sums[:, :, slot].ravel()) for slot in range(USED)]
 
 
 @pytest.mark.parametrize("missing", ["all", "one", "high", "low"])
