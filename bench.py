@@ -296,7 +296,7 @@ def run_ours(args: argparse.Namespace) -> dict | None:
         device_ms = float(t.item())
     # Per-kernel device times (separate pass with events between kernels).
     timed(max(1, min(args.steps, 20)), True)
-    per_kernel = {KERNEL_NAMES[k]: kernel_ms[k] for k in range(int(kernels.value))}
+    per_kernel = {name: kernel_ms[k] for k, name in enumerate(KERNEL_NAMES)}
     per_kernel_launches = max(1, min(args.steps, 20))
     result = lsm_call_result(request.exercise_rows)
     st = lib.fo_lsm_call_plan_collect(plan, ctypes.byref(result.struct), ctypes.byref(err))
@@ -355,7 +355,7 @@ def run_ours(args: argparse.Namespace) -> dict | None:
     # The diagnostic runs on a side stream beside the backward pass: it is timed on its own stream
     # and left out of the shares of the serial kernel chain.
     serial_ms = sum(v for k, v in per_kernel.items() if k != "diagnose_kernel")
-    for name in KERNEL_NAMES[: int(kernels.value)]:
+    for name in KERNEL_NAMES:
         ms = per_kernel[name] / per_kernel_launches
         bytes_per_launch = algorithmic if name in PATH_DATA_KERNELS else 0
         roofline_all[name] = {
@@ -398,7 +398,7 @@ def run_ours(args: argparse.Namespace) -> dict | None:
             "d2h_bytes_per_step": int(d2h.value),
             "api": "finoptions.price_lsm_call(executor=CudaExecutor)",
         },
-        "gpu_launches": (int(kernels.value) + 1) * args.steps,  # the timed kernels and the reset before them
+        "gpu_launches": int(kernels.value) * args.steps,
         "roofline": {
             "kernel": dominant,
             # The backward pass is bound by the latency of its 52 dependent row exchanges, not by HBM: achieved / peak below is its

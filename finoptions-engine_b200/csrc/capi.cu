@@ -418,15 +418,22 @@ Error plan_launch(fo_lsm_call_plan* plan) {
     return Error{};
 }
 
-// Kernels of one launch, each a timed segment.
-uint64_t kernels_per_launch(const fo_lsm_call_plan* plan) { return plan->run_eval ? 5 : 4; }
+// Timed segments of one launch: simulate, moments, backward, diagnose and, where it runs, evaluate.
+uint64_t segments_per_launch(const fo_lsm_call_plan* plan) { return plan->run_eval ? 5 : 4; }
+
+// Kernels of one launch: reset, simulate, the moments' (one or two), backward, diagnose, evaluate.
+uint64_t kernels_per_launch(const fo_lsm_call_plan* plan) {
+    const HostPlan& hp = plan->hp;
+    const uint64_t moments = fitted_rows(hp) > 0 ? uint64_t(moment_launches(hp.train_paths, hp.degree)) : 0;
+    return 3 + moments + (hp.rows() > 1 ? 1 : 0) + (plan->run_eval ? 1 : 0);
+}
 
 Error plan_time_launches(fo_lsm_call_plan* plan, uint32_t iterations, double* elapsed_ms, double* kernel_ms,
                          uint64_t capacity) {
     cudaStream_t s = plan->ex->stream;
     for (cudaEvent_t& e : plan->marks)
         if (!e) FO_CUDA_TRY(cudaEventCreate(&e), "cudaEventCreate");
-    const uint64_t kernels = kernels_per_launch(plan);
+    const uint64_t kernels = segments_per_launch(plan);
     std::vector<double> sums(kernels, 0.0);
     cudaEvent_t begin = plan->marks[8], end = plan->marks[9];
     // Segments in the order simulate, moments, backward, diagnose, evaluate. The diagnostic runs beside

@@ -562,6 +562,8 @@ int moment_blocks(uint64_t paths, uint32_t rows, int sms, size_t workspace_bytes
 
 size_t moment_workspace_bytes(uint32_t rows, int blocks) { return sizeof(double2) * kSlots * rows * size_t(blocks); }
 
+int moment_launches(uint64_t paths, int degree) { return degree > 0 && paths > kRetakePaths ? 2 : 1; }
+
 template <int D>
 static cudaError_t launch_moments_d(const MomentArgs& args, int rows, int blocks, cudaStream_t stream) {
     // Not by launch_early: with an event recorded behind it for another stream, a call took 25 us more (52 weeks,
@@ -569,7 +571,7 @@ static cudaError_t launch_moments_d(const MomentArgs& args, int rows, int blocks
     const dim3 grid{unsigned(blocks), unsigned(rows)};
     moments_kernel<D, false><<<grid, kMomentThreads, 0, stream>>>(args);
     if constexpr (D > 0)
-        if (args.plan.train_paths > kRetakePaths) moments_kernel<D, true><<<grid, kMomentThreads, 0, stream>>>(args);
+        if (moment_launches(args.plan.train_paths, D) > 1) moments_kernel<D, true><<<grid, kMomentThreads, 0, stream>>>(args);
     return cudaGetLastError();
 }
 

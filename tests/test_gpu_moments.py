@@ -4,9 +4,13 @@ engine's contract; and the recorded means against extended precision."""
 
 from __future__ import annotations
 
+import ctypes
+
 import finoptions as fo
 import numpy as np
 import pytest
+from finoptions import _abi
+from finoptions._requests import lsm_call_request
 from test_gpu_backward_shapes import check, contract
 
 pytestmark = pytest.mark.gpu
@@ -51,3 +55,19 @@ def test_recorded_means_are_the_rounded_means_of_the_quotients(executor, strike)
         x = spots[spots > strike].astype(np.longdouble) / np.longdouble(strike)
         assert fit.in_the_money_paths == x.size
         assert abs(fit.predictor_mean - x.mean()) <= 0.55 * np.spacing(fit.predictor_mean), fit.node
+
+
+@pytest.mark.parametrize("paths, degree, exercise, kernels", [(4096, 4, 6, 6), (131072, 1, 6, 6), (131073, 1, 6, 7),
+                                                               (131073, 0, 6, 6), (131073, 4, 1, 5)])
+def test_the_kernel_count_is_what_a_launch_enqueues(native_executor, paths, degree, exercise, kernels) -> None:
+    # Reset, simulation, moments (again above 2^17 paths, where there is a pivot), backward, diagnostic, evaluation.
+    request = lsm_call_request(**{**contract(paths, degree=degree), "exercise_nodes": list(range(exercise))})
+    plan, err, count = ctypes.c_void_p(), _abi.FoError(), ctypes.c_uint64()
+    lib = _abi.load()
+    assert lib.fo_lsm_call_plan_create(native_executor.raw, ctypes.byref(request.struct), ctypes.byref(plan),
+                                       ctypes.byref(err)) == 0, err.message
+    try:
+        assert lib.fo_lsm_call_plan_kernel_count(plan, ctypes.byref(count)) == 0
+        assert count.value == kernels
+    finally:
+        lib.fo_lsm_call_plan_destroy(plan)
