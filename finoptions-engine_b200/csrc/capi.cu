@@ -117,7 +117,7 @@ Error open_device(int device, fo_executor* ex) {
 }
 
 // Chooses the persistent grid (at most one CTA per SM) and the paths per thread of the backward
-// pass. Populations up to the on-chip capacity (148 SMs x 1024 threads x the paths per thread
+// pass. Populations up to the on-chip capacity (148 SMs x 512 threads x the paths per thread
 // whose values and two spot rows fit in shared memory) keep them on chip; larger ones (*hbm) keep
 // the values in HBM and read the spots from the stored rows, on the whole grid.
 Error choose_backward_shape(const fo_executor* ex, uint64_t paths, int* blocks, int* ppt, bool* hbm) {
@@ -335,12 +335,12 @@ Error plan_launch(fo_lsm_call_plan* plan) {
     cudaStream_t s = ex->stream;
     auto* status = reinterpret_cast<DeviceStatus*>(dev + L.status);
     auto* records = reinterpret_cast<FitRecord*>(dev + L.records);
-    FO_CUDA_TRY(launch_reset(dev + L.out, L.out_bytes, status, s), "reset");
+    FO_CUDA_TRY(launch_reset(dev + L.out, L.out_bytes, status, ex->sms, s), "reset");
     auto mark = [&](int i) -> cudaError_t { return plan->timing ? cudaEventRecord(plan->marks[i], s) : cudaSuccess; };
     FO_CUDA_TRY(mark(0), "event");
     // K1 training simulation
     FO_CUDA_TRY(launch_simulate(plan->dp, plan->hp.train_paths, plan->hp.train_seed, plan->hp.train_domain, plan->d_slab,
-                                plan->first_stored_row, plan->hp.escrowed ? 1 : 0, &status->train_sim_fail, s),
+                                plan->first_stored_row, plan->hp.escrowed ? 1 : 0, &status->train_sim_fail, ex->sms, s),
                 "training simulation launch");
     FO_CUDA_TRY(mark(1), "event");
     // K2 backward induction: every row's moments, then the serial pass
@@ -927,7 +927,7 @@ Error simulate_gbm(fo_executor* executor, const fo_gbm_seeded_request& q, const 
         }
         FO_CUDA_TRY(launch_simulate_external(dp, paths, d_normals, out, &status->train_sim_fail, s), "simulation launch");
     } else {
-        FO_CUDA_TRY(launch_simulate(dp, paths, q.seed, q.domain, out, 0, 0, &status->train_sim_fail, s),
+        FO_CUDA_TRY(launch_simulate(dp, paths, q.seed, q.domain, out, 0, 0, &status->train_sim_fail, executor->sms, s),
                     "simulation launch");
     }
     unsigned long long fail = 0;

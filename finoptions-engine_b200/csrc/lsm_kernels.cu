@@ -251,22 +251,22 @@ cudaError_t launch_normals(uint64_t seed, uint32_t domain, uint32_t path_start, 
     return cudaGetLastError();
 }
 
-cudaError_t launch_reset(void* region, size_t bytes, DeviceStatus* status, cudaStream_t stream) {
+cudaError_t launch_reset(void* region, size_t bytes, DeviceStatus* status, int sms, cudaStream_t stream) {
     const size_t words = bytes / sizeof(uint4);
-    reset_kernel<<<unsigned(std::min<size_t>((words + 255) / 256, 148)), 256, 0, stream>>>(static_cast<uint4*>(region), words,
-                                                                                          status);
+    const size_t blocks = std::min<size_t>((words + 255) / 256, size_t(sms));
+    reset_kernel<<<unsigned(blocks), 256, 0, stream>>>(static_cast<uint4*>(region), words, status);
     return cudaGetLastError();
 }
 
 cudaError_t launch_simulate(const DevicePlan& plan, uint64_t paths, uint64_t seed, uint32_t domain, double* out,
                             uint32_t store_first_row, int reconstruct_escrowed, unsigned long long* fail,
-                            cudaStream_t stream) {
+                            int sms, cudaStream_t stream) {
     const int threads = kSimulateThreads;
     uint64_t blocks = (paths + threads - 1) / threads;
     // A CTA fills 15 KB of sampler tables first, about the work of eight steps: short paths share a CTA's
     // tables among several blocks of paths, down to one wave of CTAs.
     const uint64_t share = std::max<uint64_t>(1, 32 / std::max<uint32_t>(plan.intervals, 1));
-    const uint64_t wave = kSimulateCtasPerSm * 148;
+    const uint64_t wave = uint64_t(kSimulateCtasPerSm) * uint64_t(sms);
     if (blocks > wave) blocks = std::max<uint64_t>(wave, (blocks + share - 1) / share);
     if (blocks > (1u << 20)) blocks = 1u << 20;
     const auto kernel = plan.intervals <= 2 ? simulate_kernel<2> : simulate_kernel<kChunkNormals>;

@@ -93,12 +93,12 @@ cudaError_t launch_early(void (*kernel)(P...), dim3 grid, unsigned threads, size
 }
 
 // Clears a plan's read-back region (a multiple of 16 bytes), its status words to "none" where they start so.
-cudaError_t launch_reset(void* region, size_t bytes, DeviceStatus* status, cudaStream_t stream);
+cudaError_t launch_reset(void* region, size_t bytes, DeviceStatus* status, int sms, cudaStream_t stream);
 cudaError_t launch_normals(uint64_t seed, uint32_t domain, uint32_t path_start, uint64_t paths, uint32_t count,
                            double* out, unsigned long long* fail, cudaStream_t stream);
 cudaError_t launch_simulate(const DevicePlan& plan, uint64_t paths, uint64_t seed, uint32_t domain, double* out,
                             uint32_t store_first_row, int reconstruct_escrowed, unsigned long long* fail,
-                            cudaStream_t stream);
+                            int sms, cudaStream_t stream);
 cudaError_t launch_replay(const DevicePlan& plan, uint64_t seed, uint32_t domain, uint32_t path, int want_row,
                           SimFailure* out, cudaStream_t stream);
 // External normals ([intervals, paths], time-major): the first non-finite value's index, the
