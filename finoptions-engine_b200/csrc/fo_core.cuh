@@ -17,11 +17,9 @@
 
 #if defined(__CUDACC__)
 #define FO_HD __host__ __device__ __forceinline__
-#define FO_D __device__ __forceinline__
 #define FO_HD_NOINLINE static __host__ __device__ __noinline__
 #else
 #define FO_HD inline
-#define FO_D inline
 #define FO_HD_NOINLINE static inline
 #endif
 
@@ -98,7 +96,7 @@ FO_HD void philox_blocks(uint64_t block, uint32_t path, uint32_t domain, const P
 // ZIGNOR standard normals: the layer constants and bit-level conversions (lsm_normals.cuh samples).
 // ----------------------------------------------------------------------------------------------
 
-enum NormalStatus : int { kNormalOk = 0, kNormalBudget = 1, kNormalRejection = 2 };
+enum NormalStatus : int { kNormalOk = 0, kNormalRejection = 2 };
 
 constexpr int kMaxRejectionIterations = 1048576;
 constexpr uint64_t kFractionMask = (uint64_t(1) << 52) - 1;
@@ -739,9 +737,10 @@ FO_HD bool predict_continuation_d(const Model& m, double predictor, double* out)
 // intrinsic value, exact near the strike), z = d * slope + shift is the standardised moneyness
 // (spot / strike - mean) / scale, and the continuation is its polynomial in powers of z. Exercise
 // where d > 0 and d exceeds the continuation. One fma standardises and D evaluate, against three to
-// divide by the strike, three more to divide by the scale and 4 D for the basis recurrence; the
-// rounding of z is of the order of ulp(max(|z|, 1)), where that of spot / strike is magnified by
-// 1 / scale, so the continuation is at least as close to the fitted polynomial.
+// divide by the strike, three more to divide by the scale and 4 D for the basis recurrence. z is
+// within a few roundings of |z| + |shift|, where that of spot / strike is magnified by 1 / scale: against
+// the fitted polynomial in extended precision the rule's error is 0.1 to 1 times the predictor's near the
+// money and on the whole no larger far in it (volatilities of 1% to 60% a row, eight paths to thousands).
 //
 // The rule covers spots below kRuleSpotLimit of rows for which no intermediate can overflow there
 // (the bound is evaluated in make_exercise_rule). `general` marks every other row that needs more

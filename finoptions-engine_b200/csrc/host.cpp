@@ -509,7 +509,6 @@ Error build_call_plan(const fo_lsm_call_request& q, HostPlan* plan) {
 
 int32_t simulation_failure_code(int code) {
     switch (code) {
-        case kNormalBudget: return FO_CODE_RANDOM_NORMAL_BUDGET_EXHAUSTED;
         case kNormalRejection: return FO_CODE_RANDOM_NORMAL_REJECTION_LIMIT;
         default: return FO_CODE_NON_FINITE_PATH_TRANSITION;
     }
@@ -517,9 +516,6 @@ int32_t simulation_failure_code(int code) {
 
 std::string simulation_failure_message(int code, uint32_t interval, uint64_t path, double spot, double normal) {
     switch (code) {
-        case kNormalBudget:
-            return "random-normal budget exhausted at interval " + u(interval) + ", path " + u(path) +
-                   "; this indicates an internal estimator-contract violation";
         case kNormalRejection:
             return "random-normal rejection limit reached at interval " + u(interval) + ", path " + u(path) +
                    "; no variate or fallback was produced";

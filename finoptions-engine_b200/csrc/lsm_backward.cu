@@ -265,11 +265,11 @@ __device__ __forceinline__ void write_coefficients(const RowSolution& row, FitRe
 // are the same, so a path's decisions do not depend on where its value lives.
 //
 // A pass applies row k's rule to the thread's paths, discounts them to row k - 1
-// (policy.rs:1049-1063) and adds row k - 1's response sums. Between passes the first six warps
-// exchange the sums, one warp prepares the row after and one fetches its spots. Bound by the latency of the row exchanges: a row takes
-// 2.2 us at 4,096 paths (poll 0.4), 2.6 us at 65,536 (0.8) and 5.6 us at 2^20 (1.8, the pass 2.1),
-// against 9.5, 9.6 and 17.4 us when a row's moments were solved inside it, arrivals were counted and the
-// totals read by slot. 512 threads instead of 1,024 halve the per-warp reduction and keep the rule
+// (policy.rs:1049-1063) and adds row k - 1's response sums. Between passes the first eight
+// warps exchange the sums, the ninth prepares the row after and a thread of the tenth fetches its spots.
+// Bound by the latency of the row exchanges: a row takes 2.2 us at 4,096 paths (poll 0.4), 2.7 us at 65,536
+// (0.8) and 5.8 us at 2^20 (1.8, the pass 2.1), against 9.5, 9.6 and 17.4 us when a row's moments were solved
+// inside it, arrivals were counted and the totals read by slot. 512 threads instead of 1,024 halve the per-warp reduction and keep the rule
 // and the sums in registers (2^20 paths: 0.29 ms against 0.36).
 template <int D, bool kHbm>  // D == plan.degree (launch_backward dispatches on it)
 __global__ void __launch_bounds__(kBackwardThreads, 1) backward_kernel(BackwardArgs a) {

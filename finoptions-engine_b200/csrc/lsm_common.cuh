@@ -26,7 +26,7 @@ __device__ __forceinline__ void let_next_grid_start() { asm volatile("griddepcon
 // ---------------------------------------------------------------------------------------------
 
 struct SimResult {
-    int code;  // 0 ok, kNormalBudget, kNormalRejection, 3 non-finite transition
+    int code;  // 0 ok, kNormalRejection, 3 non-finite transition
     int interval;
     double spot;
     double normal;

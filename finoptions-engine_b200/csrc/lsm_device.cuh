@@ -75,7 +75,7 @@ constexpr size_t kStatusNoneBytes = 7 * sizeof(unsigned long long) + sizeof(unsi
 // Failure replay record for one path (filled by the replay kernel): the failure, if any, and
 // the state observed at one requested row.
 struct SimFailure {
-    int32_t code;      // 0 none, kNormalBudget, kNormalRejection, or 3 = non-finite transition
+    int32_t code;      // 0 none, kNormalRejection, or 3 = non-finite transition
     int32_t interval;
     double spot;
     double normal;

@@ -32,8 +32,10 @@ using namespace fo;
 namespace {
 
 constexpr unsigned long long kNone = ~0ull;
-// Shared memory the persistent launch may spend on staged fitted rules (with three 80-register
-// CTAs per SM, about 57 KB each leaves every CTA resident; more lowers the CTAs per SM).
+// Shared memory an evaluation may spend on staged rules beside the 40 to 47 KB of its kernel's own (227 KB a CTA at
+// most). Eight strikes' rules of up to 55 rows leave the persistent launch its three CTAs per SM, of up to 145 rows
+// the phase executor's evaluation its two; up to 317 rows (and 2,400 of one strike) they are still staged,
+// with fewer CTAs.
 constexpr size_t kPersistentRuleSmemBytes = 160 * 1024;
 constexpr uint32_t kGreekRuleRows = 1462;  // observation rows of a contract priced with its Greeks
 constexpr int kPersistentMaxCtasPerSm = 3;  // the persistent kernel's launch bounds
@@ -1577,8 +1579,10 @@ Error price_groups(fo_executor* ex, const BatchMethod& m, const std::vector<Grou
                 // External record nodes: the marks are recorded when the graph runs (a plain record
                 // during capture would only order the captured work).
                 if (ce == cudaSuccess) ce = cudaEventRecordWithFlags(mark[0], s, cudaEventRecordExternal);
+                // Simulation, fits and evaluation drain a queue each; the diagnostics and the summaries take none.
+                constexpr int phase_queue[kBatchPhaseLaunches] = {0, 1, 2, 2, 2};
                 for (int k = 0; k < n_launches && ce == cudaSuccess; ++k) {
-                    ce = enqueue_batch_persistent(launch[k], a, tune.phases ? qs[k < 2 ? k : 2] : q, max_rows, stage, s);
+                    ce = enqueue_batch_persistent(launch[k], a, tune.phases ? qs[phase_queue[k]] : q, max_rows, stage, s);
                     if (ce == cudaSuccess) ce = cudaEventRecordWithFlags(mark[k + 1], s, cudaEventRecordExternal);
                 }
                 if (ce == cudaSuccess) ce = cudaMemcpyAsync(back, dev + L.out_begin, L.out_bytes, cudaMemcpyDeviceToHost, s);

@@ -110,7 +110,7 @@ struct NormalStream {
         for (uint32_t j = 0; j < C; ++j) z[j] = ring[((k + j) % kRing) * T];
         return true;
     }
-    // Normal k of the chunk that next4 handed out last.
+    // Normal k of the chunk that next handed out last.
     __device__ __forceinline__ double normal(uint32_t k) const { return ring[(k % kRing) * T]; }
 
     // N blocks through the sampler.

@@ -222,8 +222,8 @@ __device__ __forceinline__ double load_slab(const double* p) {
 // of L2 traffic, and between two rows' passes stands a serial part (reduce, decide, fit, rule) of 13,000
 // cycles that only the SM's other CTA can fill. At 4,096 states x 8 strikes x 32,768 paths the fits took
 // 271 ms with four CTAs per SM, one path at a time and every value in HBM, its paths decided in a branch of
-// their own. They take 167 ms so: two CTAs (128 registers a thread; with three or four the pass spills, 197
-// and 274 ms), values on chip where they fit, kU = 4 paths side by side without a branch (kU = 2 179 ms,
+// their own. They take 167 ms so: two CTAs (128 registers a thread, 176 bytes of spill stores in the kernel; with three or
+// four the pass spills, 197 and 274 ms), values on chip where they fit, kU = 4 paths side by side without a branch (kU = 2 179 ms,
 // 3 167 ms) and the next four loaded ahead (170 ms without). A row takes 75,000 cycles, 58,000 the pass.
 template <int D, bool kReadOnlySlab, bool kTeam, int kU>
 __device__ bool backward_item(const BatchArgs& a, uint32_t pi, uint32_t member, uint32_t members, unsigned* timeout,
@@ -1066,7 +1066,8 @@ constexpr int kFitCtasPerSm = 2;
 template <int kPhase, int S, bool kGreeks>
 struct PhaseOccupancy {
     // Resident CTAs per SM the register budget is cut for. The adjoint's at four took 58.1 ms for 1,024
-    // ragged contracts, its state spilled; at three 48.7, at two 52.3.
+    // ragged contracts, its state spilled; at three 48.7, at two 52.3. The one-strike evaluation spills 424
+    // bytes at its four.
     static constexpr int value = kPhase == kPhaseSimulate               ? 4
                                  : kPhase == kPhaseFit                  ? kFitCtasPerSm
                                  : kPhase == kPhaseEvaluate && kGreeks  ? 3
