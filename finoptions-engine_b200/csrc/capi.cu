@@ -175,6 +175,35 @@ PlanLayout layout_for(const HostPlan& hp, int backward_blocks, int eval_blocks, 
 // Rows whose moments are reduced ahead of the backward pass.
 uint32_t fitted_rows(const HostPlan& hp) { return hp.rows() - 1 - (hp.origin_row ? 1u : 0u); }
 
+// Whether a second moments launch follows for rows whose pivot was too far (lsm_backward.cu): one CTA reads
+// kRetakePaths paths again in 80 us, where the launch takes 4. Only rows with few in-the-money paths among the
+// thousand that set the pivot come to that, so it takes a fitted row whose median, on the way to which the cash
+// dividends are paid, lies more than 1.5 standard deviations below the strike (7% in the money). A row
+// missed here (cash that is not always paid) is summed again by its last CTA, which is only slower.
+constexpr uint64_t kRetakePaths = 1 << 17;
+bool moments_relaunch(const HostPlan& hp) {
+    if (hp.train_paths <= kRetakePaths || hp.degree == 0) return false;
+    const double strike = std::log(hp.strike);
+    const uint32_t last = hp.rows() - 1;
+    double level = std::log(hp.sim_start), variance = 0.0;
+    for (uint32_t i = 0; i < hp.intervals(); ++i) {
+        level += hp.steps[i].log_drift;
+        variance += hp.steps[i].diffusion * hp.steps[i].diffusion;
+        const NodeEvent& ev = hp.events[i + 1];
+        if (ev.row >= 0 && uint32_t(ev.row) < last) {
+            const double median = hp.escrowed ? std::log(std::exp(level) + hp.escrow_cash[ev.row]) : level;
+            const double above = strike - median;
+            if (above > 0.0 && above * above > 2.25 * variance) return true;
+        }
+        if (ev.flags & kEventDividend) {
+            const double paid = std::exp(level) - ev.dividend_amount;
+            if (!(paid > 0.0)) return true;
+            level = std::log(paid);
+        }
+    }
+    return false;
+}
+
 // Workspace in which every CTA of the moments launch finds room for its totals (none with one CTA a row).
 // A small evaluation beside a large training population has fewer partials of its own: 12 dates, 3,000,001
 // training and 4,096 evaluation paths took 1,985 us a call with the CTAs that fit among those.
@@ -354,6 +383,7 @@ Error plan_launch(fo_lsm_call_plan* plan) {
     mo.exchange_words = exchange_words(plan->backward_blocks);
     if (const uint32_t rows = fitted_rows(plan->hp); rows > 0) {
         const int blocks = moment_blocks(plan->hp.train_paths, rows, ex->sms, L.workspace_bytes);
+        mo.relaunch = moments_relaunch(plan->hp) ? 1 : 0;
         FO_CUDA_TRY(launch_moments(mo, blocks, s), "moments launch");
     } else {
         FO_CUDA_TRY(cudaMemsetAsync(mo.exchange, 0, sizeof(double2) * mo.exchange_words, s), "reset");
@@ -424,7 +454,7 @@ uint64_t segments_per_launch(const fo_lsm_call_plan* plan) { return plan->run_ev
 // Kernels of one launch: reset, simulate, the moments' (one or two), backward, diagnose, evaluate.
 uint64_t kernels_per_launch(const fo_lsm_call_plan* plan) {
     const HostPlan& hp = plan->hp;
-    const uint64_t moments = fitted_rows(hp) > 0 ? uint64_t(moment_launches(hp.train_paths, hp.degree)) : 0;
+    const uint64_t moments = fitted_rows(hp) > 0 ? (moments_relaunch(hp) ? 2 : 1) : 0;
     return 3 + moments + (hp.rows() > 1 ? 1 : 0) + (plan->run_eval ? 1 : 0);
 }
 

@@ -50,15 +50,14 @@ __device__ __forceinline__ double moneyness(double spot, const Divisor& strike) 
 // CTA totals in order, solves the row (lsm_fit_warp.cuh with zero responses) and writes its record.
 // The power sums are taken about the in-the-money mean of the row's first thousand paths, which
 // lies within a fraction of a standard deviation of the row's. Where it does not (a few in-the-money
-// paths), the row's sums are taken again about its own mean: by the last CTA alone, or, for more than
-// kRetakePaths paths, by a second launch (kAgain), whose CTAs leave at once for every other row. 52
-// weeks, 2^20 paths, strike at 1.6 times the spot: 1,906 us a call by the last CTA, 1,308 so.
+// paths), the row's sums are taken again about its own mean: by the last CTA alone, or by a second
+// launch (kAgain) where the caller announced one, whose CTAs leave at once for every other row. 52 weeks, 2^20
+// paths, strike at 1.6 times the spot: 1,906 us a call by the last CTA, 1,308 so.
 // It reads the stored rows once, at about half the FP64 rate and half of HBM's: 2^20 paths x 51 rows take
 // 143 us, 200 us with every power added by itself.
 constexpr int kMomentThreads = 256;
 constexpr int kMomentCtasPerSm = 4;
 constexpr int kPivotLoads = 4;  // the pivot's sample: the row's first kPivotLoads * kMomentThreads paths
-constexpr uint64_t kRetakePaths = 1 << 17;  // one CTA reads this many in 80 us, the second launch takes 4
 constexpr int kHugeSlot = kBadSlot + 1;  // in-the-money paths beyond kRuleSpotLimit
 
 // A path's t is its correctly rounded quotient by the strike less the pivot. (One fma with the strike's
@@ -185,7 +184,7 @@ __global__ void __launch_bounds__(kMomentThreads, kMomentCtasPerSm) moments_kern
     double mean = pivot;
     if (!kAgain && D > 0 && population >= required && bad == 0 && pivot_too_far(total, pivot, itm, &mean)) {
         pivot = mean;
-        if (P > kRetakePaths) {
+        if (a.relaunch) {
             if (threadIdx.x == 0) {
                 rec.pivot = pivot;
                 rec.arrived = 0;
@@ -562,8 +561,6 @@ int moment_blocks(uint64_t paths, uint32_t rows, int sms, size_t workspace_bytes
 
 size_t moment_workspace_bytes(uint32_t rows, int blocks) { return sizeof(double2) * kSlots * rows * size_t(blocks); }
 
-int moment_launches(uint64_t paths, int degree) { return degree > 0 && paths > kRetakePaths ? 2 : 1; }
-
 template <int D>
 static cudaError_t launch_moments_d(const MomentArgs& args, int rows, int blocks, cudaStream_t stream) {
     // Not by launch_early: with an event recorded behind it for another stream, a call took 25 us more (52 weeks,
@@ -571,7 +568,7 @@ static cudaError_t launch_moments_d(const MomentArgs& args, int rows, int blocks
     const dim3 grid{unsigned(blocks), unsigned(rows)};
     moments_kernel<D, false><<<grid, kMomentThreads, 0, stream>>>(args);
     if constexpr (D > 0)
-        if (moment_launches(args.plan.train_paths, D) > 1) moments_kernel<D, true><<<grid, kMomentThreads, 0, stream>>>(args);
+        if (args.relaunch) moments_kernel<D, true><<<grid, kMomentThreads, 0, stream>>>(args);
     return cudaGetLastError();
 }
 

@@ -24,6 +24,7 @@ struct MomentArgs {
     DeviceStatus* status;
     double2* exchange;           // BackwardArgs::partials
     int exchange_words;          // exchange_words(backward blocks)
+    int relaunch;                // a second launch takes the rows again whose pivot was too far
 };
 
 struct BackwardArgs {
@@ -111,7 +112,6 @@ cudaError_t launch_replay_external(const DevicePlan& plan, uint64_t paths, const
 // CTAs per row of the moments launch, at most what the workspace holds; what that many take.
 int moment_blocks(uint64_t paths, uint32_t rows, int sms, size_t workspace_bytes);
 size_t moment_workspace_bytes(uint32_t rows, int blocks);
-int moment_launches(uint64_t paths, int degree);
 cudaError_t launch_moments(const MomentArgs& args, int blocks, cudaStream_t stream);
 int backward_max_blocks(int device);
 int backward_max_ppt();

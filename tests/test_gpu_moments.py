@@ -57,11 +57,14 @@ def test_recorded_means_are_the_rounded_means_of_the_quotients(executor, strike)
         assert abs(fit.predictor_mean - x.mean()) <= 0.55 * np.spacing(fit.predictor_mean), fit.node
 
 
-@pytest.mark.parametrize("paths, degree, exercise, kernels", [(4096, 4, 6, 6), (131072, 1, 6, 6), (131073, 1, 6, 7),
-                                                               (131073, 0, 6, 6), (131073, 4, 1, 5)])
-def test_the_kernel_count_is_what_a_launch_enqueues(native_executor, paths, degree, exercise, kernels) -> None:
-    # Reset, simulation, moments (again above 2^17 paths, where there is a pivot), backward, diagnostic, evaluation.
-    request = lsm_call_request(**{**contract(paths, degree=degree), "exercise_nodes": list(range(exercise))})
+@pytest.mark.parametrize("paths, strike, degree, exercise, kernels", [
+    (4096, 100.0, 4, 6, 6), (131072, 160.0, 1, 6, 6), (131073, 160.0, 1, 6, 7), (131073, 100.0, 1, 6, 6),
+    (131073, 160.0, 0, 6, 6), (131073, 160.0, 4, 1, 5)])
+def test_the_kernel_count_is_what_a_launch_enqueues(native_executor, paths, strike, degree, exercise, kernels) -> None:
+    # Reset, simulation, moments (again for far strikes above 2^17 paths, where there is a pivot), backward,
+    # diagnostic, evaluation.
+    request = lsm_call_request(**{**contract(paths, strike=strike, degree=degree),
+                                  "exercise_nodes": list(range(exercise))})
     plan, err, count = ctypes.c_void_p(), _abi.FoError(), ctypes.c_uint64()
     lib = _abi.load()
     assert lib.fo_lsm_call_plan_create(native_executor.raw, ctypes.byref(request.struct), ctypes.byref(plan),
