@@ -608,8 +608,8 @@ int backward_max_blocks(int device) {
 template <int D, bool kHbm>
 static cudaError_t launch_backward_d(const BackwardArgs& args, int blocks, int ppt, cudaStream_t stream) {
     const size_t smem = kHbm ? 0 : backward_smem_bytes(ppt);
-    cudaError_t e = cudaFuncSetAttribute(backward_kernel<D, kHbm>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         int(smem));
+    const cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void*>(backward_kernel<D, kHbm>), smem,
+                                             sizeof(BackwardSmem) + 256);
     if (e != cudaSuccess) return e;
     // The launch itself refuses a grid that cannot be resident (cudaErrorCooperativeLaunchTooLarge).
     void* params[] = {const_cast<BackwardArgs*>(&args)};

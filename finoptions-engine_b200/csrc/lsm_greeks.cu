@@ -131,10 +131,8 @@ static cudaError_t launch_evaluate_greeks_d(const EvalArgs& args, const GreeksAr
     const size_t smem = evaluate_greeks_smem_bytes(args.plan.rows);
     const auto kernel =
         args.plan.intervals <= 2 ? evaluate_greeks_kernel<D, 2> : evaluate_greeks_kernel<D, kChunkNormals>;
-    if (smem > kSmallDynamicSmem) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-        if (e != cudaSuccess) return e;
-    }
+    const cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
+    if (e != cudaSuccess) return e;
     return launch_early(kernel, dim3(unsigned(blocks)), kEvalThreads, smem, stream, args, greeks);
 }
 

@@ -320,10 +320,8 @@ size_t evaluate_smem_bytes(uint32_t rows) {
 template <int D>
 static cudaError_t launch_evaluate_d(const EvalArgs& args, int blocks, size_t smem, cudaStream_t stream) {
     const auto kernel = args.plan.intervals <= 2 ? evaluate_kernel<D, 2> : evaluate_kernel<D, kChunkNormals>;
-    if (smem > kSmallDynamicSmem) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-        if (e != cudaSuccess) return e;
-    }
+    const cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void*>(kernel), smem, sizeof(NormalSmem<kEvalThreads>) + 1024);
+    if (e != cudaSuccess) return e;
     return launch_early(kernel, dim3(unsigned(blocks)), kEvalThreads, smem, stream, args);
 }
 

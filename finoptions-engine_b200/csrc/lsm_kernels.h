@@ -11,10 +11,6 @@ namespace fo {
 
 constexpr int kBackwardThreads = 512;
 constexpr int kEvalThreads = 256;
-// Dynamic shared memory that fits beside any kernel's static shared memory without opting in to more
-// than 48 KB a CTA.
-constexpr size_t kSmallDynamicSmem = 512;
-
 // The moments of every fitted row, and the backward pass's exchange buffer back at phase 0.
 struct MomentArgs {
     DevicePlan plan;
@@ -91,6 +87,24 @@ cudaError_t launch_early(void (*kernel)(P...), dim3 grid, unsigned threads, size
     config.attrs = &attribute;
     config.numAttrs = 1;
     return cudaLaunchKernelEx(&config, kernel, P(args)...);
+}
+
+// Lets a kernel take `bytes` of dynamic shared memory. The limit belongs to the kernel and not to a launch: set to
+// what each launch needs, another thread's smaller one could lower it between this one's setting and its
+// launch. So it is only ever raised, to all that a CTA has beside the kernel's static share. A kernel whose
+// static share is at most `fixed` needs no leave for what fits 48 KB with it (a query takes half a microsecond).
+inline cudaError_t allow_dynamic_smem(const void* kernel, size_t bytes, size_t fixed = 48 * 1024) {
+    if (fixed + bytes <= 48 * 1024) return cudaSuccess;
+    cudaFuncAttributes attr{};
+    cudaError_t e = cudaFuncGetAttributes(&attr, kernel);
+    if (e != cudaSuccess || size_t(attr.maxDynamicSharedSizeBytes) >= bytes) return e;
+    int device = 0, most = 0;
+    e = cudaGetDevice(&device);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+    if (e != cudaSuccess) return e;
+    if (attr.sharedSizeBytes + bytes > size_t(most)) return cudaErrorInvalidValue;
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                most - int(attr.sharedSizeBytes));
 }
 
 // Clears a plan's read-back region (a multiple of 16 bytes), its status words to "none" where they start so.

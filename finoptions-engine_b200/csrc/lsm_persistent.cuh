@@ -28,6 +28,7 @@
 #include "lsm_batch_kernels.h"
 #include "lsm_common.cuh"
 #include "lsm_fit_warp.cuh"
+#include "lsm_kernels.h"
 #include "lsm_sync.cuh"
 
 namespace fo {
@@ -1205,7 +1206,7 @@ static cudaError_t prepare_persistent_d(const BatchQueue& q, uint32_t rule_rows,
         constexpr size_t kSmBytes = 228 * 1024, kReservedPerCta = 1024, kRound = kPersistentThreads * sizeof(double);
         smem = (kSmBytes / kFitCtasPerSm - kReservedPerCta - attr.sharedSizeBytes) / kRound * kRound;
     }
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
     if (e != cudaSuccess) return e;
     int per_sm = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kPersistentThreads, smem);
